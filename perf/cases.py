@@ -31,38 +31,38 @@ VMC_TAU = 0.3
 def listed():
     return [
         # a program that makes its own moves asks for one trial move of each of a few walkers: latency
-        dict(name="ratio, 64 walkers", call="ratio", system="n2_pseudo", electrons=14, precision="fp64", walkers=64),
+        dict(name="ratio 64 walkers", call="ratio", system="n2_pseudo", electrons=14, precision="fp64", walkers=64),
         # local energies of one small set of all-electron walkers (an optimiser's or a checker's sample)
-        dict(name="evaluate, all-electron", call="evaluate", system="n2_allelectron", electrons=14, precision="fp64",
+        dict(name="evaluate all-electron", call="evaluate", system="n2_allelectron", electrons=14, precision="fp64",
              walkers=256),
         # the same for a medium molecule in mixed precision, an odd electron count and a ragged population
-        dict(name="evaluate, molecule", call="evaluate", system="molecule", electrons=43, precision="mixed",
+        dict(name="evaluate molecule", call="evaluate", system="molecule", electrons=43, precision="mixed",
              walkers=1000),
         # orbitals, gradients and Laplacians of a periodic cell on a list of points (plots, densities, fits)
-        dict(name="orbital rows, cell", call="orbitals", system="cell", electrons=128, precision="mixed", walkers=1200),
+        dict(name="orbital rows cell", call="orbitals", system="cell", electrons=128, precision="mixed", walkers=1200),
         # VMC of the all-electron molecule with the small population of an equilibration or an optimisation step
-        dict(name="vmc, all-electron", call="vmc", system="n2_allelectron", electrons=14, precision="fp64",
+        dict(name="vmc all-electron", call="vmc", system="n2_allelectron", electrons=14, precision="fp64",
              walkers=256, steps=20),
         # the headline: mixed-precision DMC of the pseudopotential molecule
-        dict(name="dmc, molecule", call="dmc", system="n2_pseudo", electrons=14, precision="mixed", walkers=4096,
+        dict(name="dmc molecule", call="dmc", system="n2_pseudo", electrons=14, precision="mixed", walkers=4096,
              steps=10, tau=0.01),
         # the same physics in FP64 on a population that is no multiple of anything
-        dict(name="dmc, molecule, fp64", call="dmc", system="n2_pseudo", electrons=14, precision="fp64", walkers=3001,
+        dict(name="dmc molecule fp64", call="dmc", system="n2_pseudo", electrons=14, precision="fp64", walkers=3001,
              steps=10, tau=0.01),
         # a few electrons and a very large population: launches, branching and copies weigh most
-        dict(name="dmc, large population", call="dmc", system="molecule", electrons=4, precision="mixed",
+        dict(name="dmc large population", call="dmc", system="molecule", electrons=4, precision="mixed",
              walkers=65536, steps=10, tau=0.01),
         # a large molecule: determinants and orbitals that no longer fit in shared memory
-        dict(name="dmc, large molecule", call="dmc", system="molecule", electrons=72, precision="mixed", walkers=2048,
+        dict(name="dmc large molecule", call="dmc", system="molecule", electrons=72, precision="mixed", walkers=2048,
              steps=5, tau=0.01),
         # a solid in FP64: Ewald sums, image sums, three-body Jastrow
-        dict(name="dmc, cell, fp64", call="dmc", system="cell", electrons=32, precision="fp64", walkers=1024, steps=5,
+        dict(name="dmc cell fp64", call="dmc", system="cell", electrons=32, precision="fp64", walkers=1024, steps=5,
              tau=0.005),
         # the same solid with twisted boundary conditions and complex orbitals
-        dict(name="dmc, cell at a k-point", call="dmc", system="kcell", electrons=32, precision="mixed", walkers=2048,
+        dict(name="dmc cell at a k-point", call="dmc", system="kcell", electrons=32, precision="mixed", walkers=2048,
              steps=5, tau=0.005),
         # the largest: a supercell of 32 atoms
-        dict(name="dmc, supercell", call="dmc", system="cell", electrons=128, precision="mixed", walkers=1024, steps=4,
+        dict(name="dmc supercell", call="dmc", system="cell", electrons=128, precision="mixed", walkers=1024, steps=4,
              tau=0.005),
     ]
 
