@@ -119,7 +119,7 @@ struct qwg_ctx {
   bool own_stream = false;
   long long launches = 0;
   // tables
-  DevBuf d_shell_i, d_shell_obj, d_shell_cut, d_spline, d_spline64, d_moc, d_moc_im, d_image_kfac;
+  DevBuf d_shell_i, d_shell_obj, d_shell_cut, d_shell_order, d_spline, d_spline64, d_moc, d_moc_im, d_image_kfac;
   DevBuf d_image_pos, d_gvec, d_gweight, d_ion_sin, d_ion_cos;
   DevBuf d_sub_seg, d_sub_idx;  // sub-cell candidate lists of the image sums
   int sub_n[3] = {0, 0, 0};
@@ -206,6 +206,7 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
   S.shell_i = c->d_shell_i.as<int4>();
   S.shell_obj = c->d_shell_obj.as<int2>();
   S.shell_cut = c->d_shell_cut.as<double>();
+  S.shell_order = c->d_shell_order.as<int>();
   S.spline = c->d_spline.as<Real>();
   S.spline64 = c->d_spline64.as<double>();
   S.moc = c->d_moc.as<Real>();
@@ -251,6 +252,17 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
     if (sh.first >= (1 << 16) || sh.k >= 256) throw InputError("basis too large for the shell table");
     S.shell_pack[k] = sh.sym | (sh.first << 4) | (sh.k << 20);
   }
+  // centers of a cell with S and P shells only: S first, then P (each in
+  // object order), so that the image sums can keep them in registers
+  if (H.periodic && !H.cutoff_mo)
+    for (int a = 0; a < H.natoms; a++) {
+      const int4 cs = S.center_seg[a];
+      int* first = S.shell_pack + cs.x;
+      const auto sym = [](int pack) { return pack & 0xf; };
+      if (cs.y == 0 || std::any_of(first, first + cs.y, [&](int k) { return sym(k) > 1; })) continue;
+      const int* p = std::stable_partition(first, first + cs.y, [&](int k) { return sym(k) == 0; });
+      S.center_sp[a] = make_int2((int)(p - first), cs.y - (int)(p - first));
+    }
   // periodic cell and basis image centers
   S.periodic = H.periodic ? 1 : 0;
   for (int i = 0; i < 3; i++) {
@@ -445,6 +457,11 @@ static void build_tables(qwg_ctx* c) {
   upload(c->d_shell_i, si, st);
   upload(c->d_shell_obj, so, st);
   upload(c->d_shell_cut, sc, st);
+  // image sums: the shells by shape
+  std::vector<int> order(H.shells.size());
+  for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return H.shells[a].sym > H.shells[b].sym; });
+  upload(c->d_shell_order, order, st);
   // MO coefficients padded to the orbital stride, both spins
   const int mm = mo_stride_for(c->mmax, std::max(H.nmo[0], H.nmo[1]));
   std::vector<double> moc((size_t)2 * H.nbasis * mm, 0.0), moc_im(moc.size(), 0.0);
@@ -660,7 +677,7 @@ static size_t footprint_bytes(const qwg_ctx* c, int max_walkers) {
   for (size_t o = 0; o < H.obj_first.size(); o++) total4 += (size_t)H.spline_npts * H.obj_count[o];
   const size_t ms = mo_stride_for(c->mmax, std::max(H.nmo[0], H.nmo[1]));
   const size_t cf = c->mmax == kComplexFamily ? 2 : 1;
-  size_t b = total4 * 4 * (8 + rs) + 2 * (size_t)H.nbasis * ms * rs * cf + H.shells.size() * 32 +
+  size_t b = total4 * 4 * (8 + rs) + 2 * (size_t)H.nbasis * ms * rs * cf + H.shells.size() * 36 +
              H.image_pos.size() * 8 * 5 / 3 + H.gvec.size() * 8 + 3 * H.gweight.size() * 8;
   if (H.periodic) {
     const SubcellLists sl = make_subcell_lists(H);

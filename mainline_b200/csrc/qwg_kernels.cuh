@@ -46,7 +46,8 @@ struct PPItem {
 // XL: the F/G-shell and CUTOFF_MO code (HBM-resident kernels; the FP32 ones
 // are also compiled without it for the decks that need none, as that code's
 // register demand costs the move kernel ~5% in spills).
-template <typename Real, int MMAX, bool TB, int PER, bool XL = (MMAX <= 0)>
+// ROWSUM: see basis_lap_warp.
+template <typename Real, int MMAX, bool TB, int PER, bool XL = (MMAX <= 0), bool ROWSUM = false>
 struct Walker {
   const DevSys<Real>& S;
   const WLayout& L;
@@ -158,7 +159,7 @@ struct Walker {
       double* ai = aug + (size_t)2 * M * M;
       for (int el = 0; el < M; el++) {
         const int e = e0 + el;
-        mo_lap_warp_cpx<Real>(S, mocs(s), mocs_im(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], M, ms, bas(), nc, lane);
+        mo_lap_warp_cpx<Real, ROWSUM>(S, mocs(s), mocs_im(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], M, ms, bas(), nc, lane);
         for (int i = lane; i < M; i += 32) {
           ar[el * 2 * M + i] = double(nc[i * 5]);
           ai[el * 2 * M + i] = double(nc[newcol_im_off() + i * 5]);
@@ -195,7 +196,7 @@ struct Walker {
       double* vals = mdv();
       for (int el = 0; el < M; el++) {
         const int e = e0 + el;
-        mo_lap_warp<Real, PER, HL>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], NU, bas(), nc, lane);
+        mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], NU, bas(), nc, lane);
         for (int j = lane; j < NU; j += 32) {
           vals[(size_t)el * ms + j] = double(nc[j * 5]);
           Real* mv = mov() + ((size_t)e * ms + j) * 4;
@@ -223,7 +224,7 @@ struct Walker {
       const int e0 = s == 0 ? 0 : S.nup;
       for (int el = 0; el < M; el++) {
         const int e = e0 + el;
-        mo_lap_warp<Real, PER, HL>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], M, bas(), nc, lane);
+        mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], M, bas(), nc, lane);
         for (int i = lane; i < M; i += 32) {
           aug[el * 2 * M + i] = double(nc[i * 5]);
           Real* mv = mov() + ((size_t)e * MS() + i) * 4;
@@ -320,7 +321,7 @@ struct Walker {
     if (multi()) {
       // ratios of every distinct spin-determinant (kept in mdr for accept),
       // combined with the expansion weights
-      mo_lap_warp<Real, PER, HL>(S, mocs(s), px, py, pz, S.nmo_u[s], bas(), nc, lane);
+      mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), px, py, pz, S.nmo_u[s], bas(), nc, lane);
       double* rr = mdr();
       for (int u = lane; u < S.nud[s]; u += 32) {
         const Real* iv = inv_u(s, u) + (size_t)el * MS();
@@ -344,7 +345,7 @@ struct Walker {
     } else if constexpr (CPX) {
       // complex ratio R = sum_i invT[el][i] phi_i(p); |R| returned, R kept
       // for accept; drift and Laplacian from the real parts of the ratios
-      mo_lap_warp_cpx<Real>(S, mocs(s), mocs_im(s), px, py, pz, M, MS(), bas(), nc, lane);
+      mo_lap_warp_cpx<Real, ROWSUM>(S, mocs(s), mocs_im(s), px, py, pz, M, MS(), bas(), nc, lane);
       const Real* iv = inv(s) + (size_t)el * MS();
       const Real* ivi = iv + (size_t)MS() * MS();
       const Real* nci = nc + newcol_im_off();
@@ -377,7 +378,7 @@ struct Walker {
           from_gemm = true;
         }
       }
-      if (!from_gemm) mo_lap_warp<Real, PER, HL>(S, mocs(s), px, py, pz, M, bas(), nc, lane);
+      if (!from_gemm) mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), px, py, pz, M, bas(), nc, lane);
       QWG_PHASE_END(t_mo, PH_MO, ph)
       const Real* iv = inv(s) + (size_t)el * MS();
       for (int i = 0; i < M; i++) {
@@ -896,7 +897,7 @@ struct Walker {
         } else {
           wrap_pos(S, nx, ny, nz);
           if (PER == 1 || (PER == 2 && S.periodic)) {
-            rd = basis_dot_lane_periodic<Real, HL>(S, nx, ny, nz, wr);
+            rd = basis_dot_lane_periodic<Real, HL, ROWSUM>(S, nx, ny, nz, wr);
           } else if (multi()) {
             // sum over distinct spin-determinants of T[s][u] R_u / W
             const int s = spin(I.e);
@@ -1070,7 +1071,7 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
     constexpr bool SWEEP_ONLY = mode == KM_SWEEP || mode == KM_TMOVE;  // move-phase shared memory only
     unsigned char* wb = HBM ? gstate : smem + moc_bytes + (size_t)warp * (SWEEP_ONLY ? L.sweep_bytes : L.bytes);
     unsigned char* sb = HBM ? P.scratch + (size_t)wid * L.scratch_bytes : wb + L.state_bytes;
-    Walker<Real, MMAX, TB, PER, XL> W{S, L, wb, sb, moc_s, lane};
+    Walker<Real, MMAX, TB, PER, XL, mode == KM_STEPS> W{S, L, wb, sb, moc_s, lane};
     // tensor-core move schedule: this launch moves electron P.tc_e only
     W.ph = P.phases;
     QWG_PHASE_BEGIN(t_walker)
