@@ -314,6 +314,8 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
   S.has_tb = H.tb.empty() ? 0 : 1;
   S.tb_stale_ei = H.tb_stale_ei ? 1 : 0;
   S.has_pp = H.has_pp ? 1 : 0;
+  S.tb_tab = 1;
+  S.ei_in_tb = 1;
   std::vector<int> type_done(types.size(), 0);
   for (int a = 0; a < H.natoms; a++) {
     const int t = S.atom_type[a];
@@ -333,6 +335,12 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
       S.tb[t][n] = DTB{q.k - H.ei_first[a], q.l - H.ei_first[a], q.m, q.c, q.cu};
       S.tb_rc[t] = std::max({S.tb_rc[t], S.ei[t][S.tb[t][n].k].rcut, S.ei[t][S.tb[t][n].l].rcut});
     }
+    double ei_rc = 0.0;
+    for (int k = 0; k < S.ei_n[t]; k++) ei_rc = std::max(ei_rc, S.ei[t][k].rcut);
+    S.ei_rc2[t] = ei_rc * ei_rc * (1.0 + 1e-6);
+    for (int n = 0; n < S.tb_n[t]; n++) S.tb_ee[t] |= 1 << S.tb[t][n].m;
+    if (S.ei_n[t] > QWG_TBK) S.tb_tab = 0;
+    if (ei_rc > S.tb_rc[t]) S.ei_in_tb = 0;
     const PPAtom& P = H.pp[a];
     S.pp_nchan[t] = P.nchan;
     S.pp_aip[t] = P.aip;

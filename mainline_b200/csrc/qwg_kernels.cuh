@@ -60,6 +60,10 @@ struct Walker {
   const float* tcD = nullptr;
   int tc_ldd = 0;
   unsigned long long* ph = nullptr;  // phase counters (profiling builds)
+  TBMove* tbm = nullptr;             // e-e-n tables of a proposal (TBX)
+  // e-e-n terms from tables: the HBM-resident kernels but the fused step
+  // kernel, which keeps its arithmetic (basis_lap_warp)
+  static constexpr bool TBX = TB && MMAX <= 0 && !ROWSUM;
   static constexpr bool CPX = MMAX < 0;
   // F and G basis shells and CUTOFF_MO: compiled into the HBM-resident kernels only
   static constexpr bool HL = MMAX < 0 || (MMAX == 0 && XL);
@@ -396,7 +400,12 @@ struct Walker {
     const bool se = s == 0;
     constexpr bool has3 = TB;
     NearSet nsn, nso;  // atoms in e-e-n range of the new and the old position
-    if constexpr (has3) {
+    bool tab = false;  // both in tbm with their radials
+    if constexpr (TBX) {
+      const double pn[3] = {px, py, pz}, po[3] = {ox, oy, oz};
+      tab = S.tb_tab && tb_move_tables(S, pn, po, *tbm, lane);
+    }
+    if (has3 && !tab) {
       const double pn[3] = {px, py, pz}, po[3] = {ox, oy, oz};
       near_atoms(S, pn, nsn);
       near_atoms(S, po, nso);
@@ -456,7 +465,14 @@ struct Walker {
       // gradient w.r.t. r_j of u(r_e - r_j) = -f'/r (r_e - r_j)
       double g0 = -fn * nx + fo * qx, g1 = -fn * ny + fo * qy, g2 = -fn * nz + fo * qz, l0 = ln - lo;
       if constexpr (has3) {
-        if (nsn.n >= 0 && nso.n >= 0) {
+        if (TBX && tab) {
+          const double dn[3] = {nx, ny, nz}, dq[3] = {qx, qy, qz};
+          const double rnd = sqrt(nx * nx + ny * ny + nz * nz), rqd = sqrt(qx * qx + qy * qy + qz * qz);
+          double dgj[3] = {0, 0, 0}, dlj = 0;
+          tb_pair_move_tab(S, *tbm, same, pj, dn, rnd, dq, rqd, du, ge, le, dgj, dlj);
+          g0 += dgj[0]; g1 += dgj[1]; g2 += dgj[2];
+          l0 += dlj;
+        } else if (nsn.n >= 0 && nso.n >= 0) {
           const double dn[3] = {nx, ny, nz}, dq[3] = {qx, qy, qz};
           const double rnd = sqrt(nx * nx + ny * ny + nz * nz), rqd = sqrt(qx * qx + qy * qy + qz * qz);
           double dgj[3] = {0, 0, 0}, dlj = 0;
@@ -477,8 +493,29 @@ struct Walker {
       }
       dg[0] = g0; dg[1] = g1; dg[2] = g2; dg[3] = l0;
     }
-    // one-body terms: lanes over (atom, function) pairs
-    for (int idx = lane; idx < S.natoms * QWG_MAXEI; idx += 32) {
+    // one-body terms: lanes over (atom, function) pairs, those of the tables
+    // where no function reaches beyond them
+    const bool obt = TBX && tab && S.ei_in_tb;
+    if constexpr (TBX) {
+      const int n0 = obt ? tbm->n[0] : 0, n1 = obt ? tbm->n[1] : 0;
+      for (int idx = lane; idx < (n0 + n1) * QWG_TBK; idx += 32) {
+        const int el_ = idx / QWG_TBK, k = idx - el_ * QWG_TBK;
+        const int side = el_ < n0 ? 0 : 1, q = side == 0 ? el_ : el_ - n0;
+        const int t = S.atom_type[tbm->a[side][q]];
+        if (k >= S.ei_n[t]) continue;
+        const double c = S.onebody[t][k];
+        const double* f = tbm->f[side][q][k];
+        if (side == 0) {
+          const double* d = tbm->d[0][q];
+          du += c * f[0];
+          ge[0] += c * f[1] * d[0]; ge[1] += c * f[1] * d[1]; ge[2] += c * f[1] * d[2];
+          le += c * f[2];
+        } else {
+          du -= c * f[0];
+        }
+      }
+    }
+    for (int idx = obt ? S.natoms * QWG_MAXEI : lane; idx < S.natoms * QWG_MAXEI; idx += 32) {
       const int a = idx / QWG_MAXEI, k = idx - a * QWG_MAXEI;
       const int t = S.atom_type[a];
       if (k >= S.ei_n[t]) continue;
@@ -763,7 +800,7 @@ struct Walker {
     int res_e = -1;
     // per-electron Jastrow value at the current position
     QWG_PHASE_BEGIN(t_ue)
-    for (int e = lane; e < N; e += 32)
+    for (int e = TBX ? N : lane; e < N; e += 32)  // TBX: chunk by chunk below
       Ue()[e] = double(jas_electron_val<Real, TB>(S, Rp, e, Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2]));
     __syncwarp();
     QWG_PHASE_END(t_ue, PH_PP_JASTROW, ph)
@@ -774,6 +811,19 @@ struct Walker {
     const int CH = L.wchunk;
     PPItem* it = items();
     Real* w = wproj();
+    // e-n values of the electrons for the e-e-n terms, at the end of the item
+    // list as long as the chunk's items leave that free
+    EnTable<Real> en{};
+    size_t en_at = 0;
+    bool en_ok = false;
+    if constexpr (TBX) {
+      const size_t end = sizeof(PPItem) * (size_t)CH * A, need = (size_t)N * (8 + (size_t)A * QWG_TBK * sizeof(Real));
+      if (S.tb_tab && need <= end) {
+        en_at = end - need;
+        en.val = (Real*)((unsigned char*)it + en_at);
+        en.near = (unsigned long long*)((unsigned char*)it + end - (size_t)N * 8);
+      }
+    }
     for (int e0 = 0; e0 < N; e0 += CH) {
       const int e1 = min(N, e0 + CH);
       QWG_PHASE_BEGIN(t_items)
@@ -815,7 +865,24 @@ struct Walker {
       }
       __syncwarp();
       QWG_PHASE_END(t_items, PH_PP_ITEMS, ph)
+      if constexpr (TBX) {
+        if (!en.val || nitems * sizeof(PPItem) > en_at) en_ok = false;
+        else if (!en_ok && nitems > 0) {
+          en_table_fill(S, Rp, en, lane, 32);
+          en_table_near(S, Rp, en, lane, 32);
+          en_ok = true;
+          __syncwarp();
+        }
+      }
       if (nitems == 0) continue;
+      if constexpr (TBX) {
+        for (int e = e0 + lane; e < e1; e += 32) {
+          const double* p = Rp + 3 * e;
+          Ue()[e] = double(en_ok ? jas_point_val(S, Rp, e, p[0], p[1], p[2], en)
+                                 : jas_electron_val<Real, TB>(S, Rp, e, p[0], p[1], p[2]));
+        }
+        __syncwarp();
+      }
       QWG_PHASE_BEGIN(t_proj)
       const int nproj = multi() ? L.nud : 1;  // projected-coefficient sets per electron
       for (int idx = lane; idx < (e1 - e0) * S.nbasis * nproj && multi(); idx += 32) {
@@ -912,7 +979,9 @@ struct Walker {
           }
         }
         QWG_PHASE_BEGIN(t_pj)
-        const Real u = jas_electron_val<Real, TB>(S, Rp, I.e, nx, ny, nz);
+        Real u;
+        if (TBX && en_ok) u = jas_point_val(S, Rp, I.e, nx, ny, nz, en);
+        else u = jas_electron_val<Real, TB>(S, Rp, I.e, nx, ny, nz);
         QWG_PHASE_END(t_pj, PH_PP_POINT_JAS, ph)
         double ratio = double(rd * exp(u - Real(Ue()[I.e]))) * S.pp_w[ty][q];
         // cos of the angle between the original and the quadrature direction
@@ -1072,6 +1141,10 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
     unsigned char* wb = HBM ? gstate : smem + moc_bytes + (size_t)warp * (SWEEP_ONLY ? L.sweep_bytes : L.bytes);
     unsigned char* sb = HBM ? P.scratch + (size_t)wid * L.scratch_bytes : wb + L.state_bytes;
     Walker<Real, MMAX, TB, PER, XL, mode == KM_STEPS> W{S, L, wb, sb, moc_s, lane};
+    if constexpr (TB && HBM && (mode == KM_SWEEP || mode == KM_RATIO || mode == KM_TMOVE)) {
+      __shared__ TBMove tables[4];
+      W.tbm = tables + warp;
+    }
     // tensor-core move schedule: this launch moves electron P.tc_e only
     W.ph = P.phases;
     QWG_PHASE_BEGIN(t_walker)
