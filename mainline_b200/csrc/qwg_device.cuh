@@ -86,6 +86,7 @@ struct DevSys {
   int npts;
   double spacing, inv_spacing;
   const Real* moc;               // [2][nbasis][mstride]
+  const Real* moct;              // [2][mstride][nbasis] (HBM-resident real kernels)
   // ---- parameter-bank tables
   double atom_pos[QWG_MAXA][3];
   double atom_charge[QWG_MAXA];
@@ -118,7 +119,7 @@ struct DevSys {
   // saved e-n basis only when a group has a plain THREEBODY term, so with
   // THREEBODY_SPIN alone its quadrature ratios see the stale values.
   int tb_stale_ei;
-  int tb_tab;                    // e-n functions per atom fit the e-e-n tables (QWG_TBK)
+  int en_k;                      // largest ei_n: stride of the e-n tables
   // pseudopotential per type (nchan 0: none)
   int has_pp;
   int pp_nchan[QWG_MAXT], pp_aip[QWG_MAXT];
@@ -355,6 +356,7 @@ enum QwgPhase {
 
 struct StepParams {
   int nwalk;
+  int team;             // warps per walker (HBM-resident kernels): 1, 2 or 4
   int nsteps;
   int st;               // KM_SWEEP / KM_ELOC: step of the chunk this launch performs
   int refresh;          // 1: full recompute at start, 0: load state, 2: recompute when the
@@ -468,6 +470,70 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+
+// ---------------------------------------------------------------------------
+// The threads that work on one walker: rank 0 .. size() - 1, sync() among
+// them, the sum of a value over them (the same bits in every thread).
+//
+// WarpTeam: one warp.  CtaTeam: 1, 2 or 4 warps of a CTA, decided per launch;
+// the warps meet at a named barrier of their own and exchange partial sums
+// through a double-buffered slot of shared memory, so that one barrier serves
+// a sum.
+constexpr int TEAM_SLOT = 2 * 4;  // doubles of exchange space per team
+
+struct WarpTeam {
+  int rank;
+  __device__ __forceinline__ int size() const { return 32; }
+  __device__ __forceinline__ int warp() const { return 0; }
+  __device__ __forceinline__ void sync() const { __syncwarp(); }
+  __device__ __forceinline__ double sum(double v) { return warp_sum(v); }
+  // threads of lower rank that take, and how many take in all
+  __device__ __forceinline__ int rank_among(bool take, int& total) {
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    total = __popc(m);
+    return __popc(m & ((1u << rank) - 1u));
+  }
+};
+
+struct CtaTeam {
+  int rank, n;      // threads of the team: 32, 64 or 128
+  int bar;          // named barrier
+  int flip;         // buffer of the next exchange
+  double* slot;     // [2][4]
+  __device__ __forceinline__ int size() const { return n; }
+  __device__ __forceinline__ int warp() const { return rank >> 5; }
+  __device__ __forceinline__ void sync() const {
+    if (n == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory");
+  }
+  __device__ __forceinline__ double sum(double v) {
+    v = warp_sum(v);
+    if (n == 32) return v;
+    double* s = slot + flip * 4;
+    flip ^= 1;
+    if ((rank & 31) == 0) s[warp()] = v;
+    sync();
+    double t = s[0];
+    for (int w = 1; w < n >> 5; w++) t += s[w];
+    return t;
+  }
+  __device__ __forceinline__ int rank_among(bool take, int& total) {
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    total = __popc(m);
+    int before = __popc(m & ((1u << (rank & 31)) - 1u));
+    if (n == 32) return before;
+    int* s = (int*)(slot + flip * 4);
+    flip ^= 1;
+    if ((rank & 31) == 0) s[warp()] = total;
+    sync();
+    total = 0;
+    for (int w = 0; w < n >> 5; w++) {
+      if (w < warp()) before += s[w];
+      total += s[w];
+    }
+    return before;
+  }
+};
 
 // ---------------------------------------------------------------------------
 // radial functions
@@ -758,10 +824,10 @@ __device__ __forceinline__ void add_s(O* out, double x, double y, double z, doub
 // of skipped.  Move kernel of a 32-electron cell, 1024 walkers: 13.0 -> 4.4 ms
 // in FP64, 7.1 -> 4.4 ms mixed.
 // Each sum adds the atom's images in image order, in type O.
-template <typename O, bool HL, typename Real>
-__device__ void basis_lap_images(const DevSys<Real>& S, double px, double py, double pz, O* bas, int lane) {
+template <typename O, bool HL, typename Real, class TM>
+__device__ void basis_lap_images(const DevSys<Real>& S, double px, double py, double pz, O* bas, const TM& tm) {
   const int sc = subcell_of(S, px, py, pz);
-  for (int q = lane; q < S.nshell; q += 32) {
+  for (int q = tm.rank; q < S.nshell; q += tm.size()) {
     const int s = __ldg(S.shell_order + q);
     const int4 si = S.shell_i[s];
     const int2 so = S.shell_obj[s];
@@ -835,7 +901,7 @@ __device__ void basis_lap_images(const DevSys<Real>& S, double px, double py, do
 }
 
 // Basis value, gradient and Laplacian of every basis function at one
-// position, warp-cooperative: lanes split the shells (radial spline and
+// position, by the whole team: its threads split the shells (radial spline and
 // angular factors in FP64: the Laplacian of the tight shells cancels
 // strongly); the rows go to bas [nbasis][5] in the output type O.
 // PER: 0 molecule, 1 periodic cell (compiled for that case only), 2 decided
@@ -843,17 +909,17 @@ __device__ void basis_lap_images(const DevSys<Real>& S, double px, double py, do
 // ROWSUM: image sums in the rows themselves, the code of the fused step
 // kernel: a VMC walk doubles a difference of one rounding every few moves, so
 // its kernel keeps the arithmetic, and runs keep their walks bit for bit.
-template <typename O, int PER, bool HL, bool ROWSUM = false, typename Real>
-__device__ void basis_lap_warp(const DevSys<Real>& S, double px, double py, double pz, O* bas, int lane) {
+template <typename O, int PER, bool HL, bool ROWSUM = false, typename Real, class TM>
+__device__ void basis_lap_team(const DevSys<Real>& S, double px, double py, double pz, O* bas, const TM& tm) {
   if constexpr (!ROWSUM && PER != 0) {
     if (PER == 1 || S.periodic) {
-      basis_lap_images<O, HL>(S, px, py, pz, bas, lane);
-      __syncwarp();
+      basis_lap_images<O, HL>(S, px, py, pz, bas, tm);
+      tm.sync();
       return;
     }
   }
   const int sc = PER == 0 ? -1 : subcell_of(S, px, py, pz);
-  for (int s = lane; s < S.nshell; s += 32) {
+  for (int s = tm.rank; s < S.nshell; s += tm.size()) {
     int4 si = S.shell_i[s];
     int2 so = S.shell_obj[s];
     O* b = bas + si.z * 5;
@@ -916,17 +982,17 @@ __device__ void basis_lap_warp(const DevSys<Real>& S, double px, double py, doub
             for (int c = 0; c < 5; c++) b[5 * k + c] = O(0);
     }
   }
-  __syncwarp();
+  tm.sync();
 }
 
 // MO value, gradient and Laplacian of one position, warp-cooperative: the
-// basis rows (basis_lap_warp) in bas [nbasis][5] as Real, then lanes split
+// basis rows (basis_lap_team) in bas [nbasis][5] as Real, then lanes split
 // the (MO, component) outputs of the contraction with the MO coefficients
 // moc_s [nbasis][mstride].
 template <typename Real, int PER, bool HL = false, bool ROWSUM = false>
 __device__ void mo_lap_warp(const DevSys<Real>& S, const Real* moc_s, double px, double py, double pz, int M,
                             Real* bas, Real* out, int lane) {
-  basis_lap_warp<Real, PER, HL, ROWSUM>(S, px, py, pz, bas, lane);
+  basis_lap_team<Real, PER, HL, ROWSUM>(S, px, py, pz, bas, WarpTeam{lane});
   __syncwarp();
   if (M > 32) {
     // many orbitals: lanes over MOs (coalesced coefficient rows), the basis
@@ -1167,7 +1233,7 @@ __device__ __forceinline__ void center_dot_sp(const DevSys<Real>& S, int c, cons
 // Periodic version of basis_dot_lane: each atom's functions are summed over
 // its image centers before the |value| rule and the dot with w.
 constexpr int QWG_MAXF_ATOM = 16;  // basis functions per atom on the periodic path
-// ROWSUM as in basis_lap_warp.
+// ROWSUM as in basis_lap_team.
 template <typename Real, bool HL = false, bool ROWSUM = false>
 __device__ __forceinline__ Real basis_dot_lane_periodic(const DevSys<Real>& S, double px, double py, double pz,
                                                         const Real* w) {
@@ -1255,7 +1321,7 @@ __device__ __forceinline__ void shell_radial64(const DevSys<Real>& S, int2 so, i
 // then the complex contraction with the coefficients.  Molecules have one
 // image per atom (the atom, factor 1).  bas: [nbasis][5] + imaginary plane at
 // bas + 5 nbasis; out: [M][5] + imaginary plane at out + 5 ms.
-// ROWSUM as in basis_lap_warp; otherwise the sums of an S or P shell stay in
+// ROWSUM as in basis_lap_team; otherwise the sums of an S or P shell stay in
 // registers (move kernel of a 32-electron cell at a k-point, mixed, 2048 walkers: 13.7 -> 8.1 ms).
 template <typename Real, bool ROWSUM = false>
 __device__ void mo_lap_warp_cpx(const DevSys<Real>& S, const Real* moc_re, const Real* moc_im, double px, double py,
@@ -1755,17 +1821,16 @@ __device__ void tb_pair_move(const DevSys<Real>& S, const NearSet& nsn, const Ne
 // side 1 the old) and the e-n radials there, shared by the warp's lanes: every
 // lane pairs the moved electron with another one, so the tables replace
 // QWG_NEAR x functions radials per lane by one per entry and warp.
-constexpr int QWG_TBK = 4;  // e-n functions per atom the tables hold
 struct TBMove {
   int n[2];                 // atoms in range, -1: more than QWG_NEAR
   int a[2][QWG_NEAR];
   double d[2][QWG_NEAR][3];
   double r[2][QWG_NEAR];
-  double f[2][QWG_NEAR][QWG_TBK][3];  // value, f'/r, Laplacian
+  double f[2][QWG_NEAR][QWG_MAXEI][3];  // value, f'/r, Laplacian
 };
 
 // Fills the tables for the positions p0 and p1; lanes over the atoms, then
-// over the radials.  False when a list or a type's functions do not fit.
+// over the radials.  False when a list does not hold the atoms in range.
 template <typename Real>
 __device__ bool tb_move_tables(const DevSys<Real>& S, const double p0[3], const double p1[3], TBMove& M, int lane) {
   bool fits = true;
@@ -1783,7 +1848,6 @@ __device__ bool tb_move_tables(const DevSys<Real>& S, const double p0[3], const 
           min_image(S, x, y, z);
           r = sqrt(x * x + y * y + z * z);
           in = r < S.tb_rc[t];
-          if (S.ei_n[t] > QWG_TBK) fits = false;
         }
       }
       const unsigned m = __ballot_sync(0xffffffffu, in);
@@ -1798,12 +1862,11 @@ __device__ bool tb_move_tables(const DevSys<Real>& S, const double p0[3], const 
     if (n > QWG_NEAR) fits = false;
     if (lane == 0) M.n[side] = n > QWG_NEAR ? -1 : n;
   }
-  fits = __all_sync(0xffffffffu, fits);
   __syncwarp();
   if (!fits) return false;
   const int n0 = M.n[0], n1 = M.n[1];
-  for (int idx = lane; idx < (n0 + n1) * QWG_TBK; idx += 32) {
-    const int e = idx / QWG_TBK, k = idx - e * QWG_TBK;
+  for (int idx = lane; idx < (n0 + n1) * S.en_k; idx += 32) {
+    const int e = idx / S.en_k, k = idx - e * S.en_k;
     const int side = e < n0 ? 0 : 1, q = side == 0 ? e : e - n0;
     const int t = S.atom_type[M.a[side][q]];
     if (k < S.ei_n[t]) {
@@ -1835,10 +1898,8 @@ __device__ void tb_pair_move_tab(const DevSys<Real>& S, const TBMove& M, bool sa
     const double rj2 = dj[0] * dj[0] + dj[1] * dj[1] + dj[2] * dj[2];
     if (rj2 < S.tb_rc[t] * S.tb_rc[t] * (1.0 + 1e-12)) {
       const double rj = sqrt(rj2), irj = 1.0 / rj;
-      double fj[QWG_TBK][3];
-#pragma unroll
-      for (int k = 0; k < QWG_TBK; k++)
-        if (k < S.ei_n[t]) radial_lap_ir(S.ei[t][k], rj, irj, fj[k][0], fj[k][1], fj[k][2]);
+      double fj[QWG_MAXEI][3];
+      for (int k = 0; k < S.ei_n[t]; k++) radial_lap_ir(S.ei[t][k], rj, irj, fj[k][0], fj[k][1], fj[k][2]);
       const int miss = S.tb_ee[t] & ~have;
       if (miss) {
         have |= miss;
@@ -1998,7 +2059,7 @@ __device__ T jas_electron_val(const DevSys<Real>& S, const double* R, int i, dou
 }
 
 // e-n values of every electron at every atom for the e-e-n terms of the
-// quadrature points: val[(j * natoms + a) * QWG_TBK + k], and the atoms in
+// quadrature points: val[(j * natoms + a) * en_k + k], and the atoms in
 // range of electron j as bits of near[j].  They belong to the walker, not to
 // the point, and so are taken once per walker instead of once per point.
 template <typename T>
@@ -2015,8 +2076,8 @@ __device__ void en_table_fill(const DevSys<Real>& S, const double* R, EnTable<T>
     double x = R[3 * j] - S.atom_pos[a][0], y = R[3 * j + 1] - S.atom_pos[a][1], z = R[3 * j + 2] - S.atom_pos[a][2];
     min_image(S, x, y, z);
     const T r = T(sqrt(x * x + y * y + z * z));
-    T* v = E.val + (size_t)idx * QWG_TBK;
-    for (int k = 0; k < QWG_TBK && k < S.ei_n[t]; k++) v[k] = radial_val<T>(S.ei[t][k], r);
+    T* v = E.val + (size_t)idx * S.en_k;
+    for (int k = 0; k < S.ei_n[t]; k++) v[k] = radial_val<T>(S.ei[t][k], r);
   }
 }
 // The range bits, after en_table_fill and a synchronisation (a thread per electron).
@@ -2049,7 +2110,7 @@ __device__ T jas_point_val(const DevSys<Real>& S, const double* R, int i, double
   const bool si = i < S.nup;
   int na = 0, used = 0;
   unsigned char at[QWG_NEAR];
-  T av[QWG_NEAR][QWG_TBK];
+  T av[QWG_NEAR][QWG_MAXEI];
   for (int a = 0; a < S.natoms; a++) {
     const int t = S.atom_type[a];
     double x = px - S.atom_pos[a][0], y = py - S.atom_pos[a][1], z = pz - S.atom_pos[a][2];
@@ -2076,8 +2137,8 @@ __device__ T jas_point_val(const DevSys<Real>& S, const double* R, int i, double
     if (na == QWG_NEAR) { na = -1; break; }
     at[na] = (unsigned char)a;
     used |= S.tb_ee[t];
-    for (int k = 0; k < QWG_TBK && k < S.ei_n[t]; k++)
-      av[na][k] = stale ? E.val[((size_t)i * S.natoms + a) * QWG_TBK + k] : radial_val<T>(S.ei[t][k], T(rr));
+    for (int k = 0; k < S.ei_n[t]; k++)
+      av[na][k] = stale ? E.val[((size_t)i * S.natoms + a) * S.en_k + k] : radial_val<T>(S.ei[t][k], T(rr));
     na++;
   }
   if (na < 0) return jas_electron_val<T, true>(S, R, i, px, py, pz);  // more atoms than the list holds
@@ -2102,14 +2163,11 @@ __device__ T jas_point_val(const DevSys<Real>& S, const double* R, int i, double
       const int a = at[q];
       if (!(near >> a & 1)) continue;
       const int t = S.atom_type[a];
-      const T* aj = E.val + ((size_t)j * S.natoms + a) * QWG_TBK;
-      T ajk[QWG_TBK];
-#pragma unroll
-      for (int k = 0; k < QWG_TBK; k++) ajk[k] = aj[k];
+      const T* aj = E.val + ((size_t)j * S.natoms + a) * S.en_k;
       for (int n = 0; n < S.tb_n[t]; n++) {
         const DTB& tq = S.tb[t][n];
         const T c = T(same ? tq.c : tq.cu);
-        u += c * (av[q][tq.k] * ajk[tq.l] + av[q][tq.l] * ajk[tq.k]) * ev[tq.m];
+        u += c * (av[q][tq.k] * aj[tq.l] + av[q][tq.l] * aj[tq.k]) * ev[tq.m];
       }
     }
   }

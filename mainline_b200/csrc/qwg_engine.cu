@@ -119,6 +119,7 @@ struct qwg_ctx {
   bool own_stream = false;
   long long launches = 0;
   // tables
+  DevBuf d_moct;  // MO coefficients, a row per orbital (HBM-resident kernels)
   DevBuf d_shell_i, d_shell_obj, d_shell_cut, d_shell_order, d_spline, d_spline64, d_moc, d_moc_im, d_image_kfac;
   DevBuf d_image_pos, d_gvec, d_gweight, d_ion_sin, d_ion_cos;
   DevBuf d_sub_seg, d_sub_idx;  // sub-cell candidate lists of the image sums
@@ -211,6 +212,7 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
   S.spline64 = c->d_spline64.as<double>();
   S.moc = c->d_moc.as<Real>();
   S.moc_im = c->d_moc_im.as<Real>();
+  S.moct = c->d_moct.as<Real>();
   S.image_kfac = c->d_image_kfac.as<double>();
   for (int d = 0; d < 3; d++) S.kpt[d] = H.kpt[d];
   S.kint = 1;
@@ -314,7 +316,6 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
   S.has_tb = H.tb.empty() ? 0 : 1;
   S.tb_stale_ei = H.tb_stale_ei ? 1 : 0;
   S.has_pp = H.has_pp ? 1 : 0;
-  S.tb_tab = 1;
   S.ei_in_tb = 1;
   std::vector<int> type_done(types.size(), 0);
   for (int a = 0; a < H.natoms; a++) {
@@ -339,7 +340,7 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
     for (int k = 0; k < S.ei_n[t]; k++) ei_rc = std::max(ei_rc, S.ei[t][k].rcut);
     S.ei_rc2[t] = ei_rc * ei_rc * (1.0 + 1e-6);
     for (int n = 0; n < S.tb_n[t]; n++) S.tb_ee[t] |= 1 << S.tb[t][n].m;
-    if (S.ei_n[t] > QWG_TBK) S.tb_tab = 0;
+    S.en_k = std::max(S.en_k, S.ei_n[t]);
     if (ei_rc > S.tb_rc[t]) S.ei_in_tb = 0;
     const PPAtom& P = H.pp[a];
     S.pp_nchan[t] = P.nchan;
@@ -480,6 +481,14 @@ static void build_tables(qwg_ctx* c) {
         moc_im[((size_t)s * H.nbasis + f) * mm + i] = H.moc_im[s][(size_t)f * H.nmo[s] + i];
       }
   if (c->mmax != kComplexFamily) moc_im.clear();
+  std::vector<double> moct;
+  if (c->mmax == 0) {
+    moct.resize((size_t)2 * mm * H.nbasis, 0.0);
+    for (int s = 0; s < 2; s++)
+      for (int i = 0; i < H.nmo[s]; i++)
+        for (int f = 0; f < H.nbasis; f++)
+          moct[((size_t)s * mm + i) * H.nbasis + f] = H.moc[s][(size_t)f * H.nmo[s] + i];
+  }
   // determinant expansion: weights, (up, down) spin-determinant of each
   // determinant, union columns of every distinct spin-determinant
   upload(c->d_det_c, H.detwt, st);
@@ -494,6 +503,7 @@ static void build_tables(qwg_ctx* c) {
     upload(c->d_spline, il, st);
     upload(c->d_moc, moc, st);
     upload(c->d_moc_im, moc_im, st);
+    upload(c->d_moct, moct, st);
   } else {
     std::vector<float> sf(il.begin(), il.end());
     std::vector<float> mf(moc.begin(), moc.end());
@@ -501,6 +511,7 @@ static void build_tables(qwg_ctx* c) {
     upload(c->d_spline, sf, st);
     upload(c->d_moc, mf, st);
     upload(c->d_moc_im, mfi, st);
+    upload(c->d_moct, std::vector<float>(moct.begin(), moct.end()), st);
   }
   upload(c->d_image_pos, H.image_pos, st);
   // k-point factor of every image center: e^{i pi k.n} (complex orbitals) or
@@ -684,8 +695,7 @@ static size_t footprint_bytes(const qwg_ctx* c, int max_walkers) {
   size_t total4 = 0;
   for (size_t o = 0; o < H.obj_first.size(); o++) total4 += (size_t)H.spline_npts * H.obj_count[o];
   const size_t ms = mo_stride_for(c->mmax, std::max(H.nmo[0], H.nmo[1]));
-  const size_t cf = c->mmax == kComplexFamily ? 2 : 1;
-  size_t b = total4 * 4 * (8 + rs) + 2 * (size_t)H.nbasis * ms * rs * cf + H.shells.size() * 36 +
+  size_t b = total4 * 4 * (8 + rs) + 2 * (size_t)H.nbasis * ms * rs * (hbm_family(c->mmax) ? 2 : 1) + H.shells.size() * 36 +
              H.image_pos.size() * 8 * 5 / 3 + H.gvec.size() * 8 + 3 * H.gweight.size() * 8;
   if (H.periodic) {
     const SubcellLists sl = make_subcell_lists(H);
@@ -714,9 +724,29 @@ static void ensure_smem_attr(K kern, size_t bytes) {
   }
 }
 
+// Warps per walker of the HBM-resident kernels whose work is independent over
+// electrons, points or shells (the local energy, the evaluation, the basis
+// rows of the tensor-core schedule).  A warp per walker leaves the GPU (16
+// resident warps per SM) part empty below kWarpSlots walkers and a walker of
+// many electrons waiting on itself; two warps meet too rarely to cost more
+// than a few per cent.  Measured with 1 / 2 / 4 warps: local energy of a
+// 32-electron cell, FP64, 1024 walkers 7.6 / 5.3 / 5.3 ms, 4096 walkers 19.3 /
+// 18.5 / 17.8 ms; 128-electron cell, mixed, 1024 walkers 32.9 / 20.9 / 20.7
+// ms; 72-electron molecule, mixed, 2048 walkers 5.7 / 5.2 / 5.1 ms; a
+// 20-electron molecule, mixed, 4096 walkers 0.59 / 0.61 / 0.66 ms; evaluation
+// of a 43-electron molecule, mixed, 1000 walkers (its recompute is one warp's
+// work) 4.9 / 3.7 / 4.1 ms.
+constexpr int kWarpSlots = 148 * 16;
+static int team_warps(const qwg_ctx* c, int mode, const StepParams& P, int nwalk) {
+  if (!(mode == KM_ELOC || mode == KM_ELOC_TM || mode == KM_EVAL || (mode == KM_SWEEP && P.tc_phase == 1))) return 1;
+  if (4 * nwalk <= kWarpSlots) return 4;
+  return nwalk < kWarpSlots || c->H.nelec >= 32 ? 2 : 1;
+}
+
 template <typename Real, int MM>
-static void launch_walkers_t(qwg_ctx* c, const DevSys<Real>& S, const StepParams& P, const EvalIO& io, int mode,
+static void launch_walkers_t(qwg_ctx* c, const DevSys<Real>& S, StepParams P, const EvalIO& io, int mode,
                              int nwalk) {
+  P.team = hbm_family(MM) ? team_warps(c, mode, P, nwalk) : 1;
   const bool sw = mode == KM_SWEEP || mode == KM_TMOVE;  // move-phase shared-memory layout
   CK((launch_walker_kernels<Real, MM>(S, c->L, P, io, mode, nwalk, sw ? c->wpc_sweep : c->wpc,
                                       sw ? c->smem_sweep : c->smem_bytes, c->stream)));

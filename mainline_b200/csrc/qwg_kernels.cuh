@@ -46,8 +46,9 @@ struct PPItem {
 // XL: the F/G-shell and CUTOFF_MO code (HBM-resident kernels; the FP32 ones
 // are also compiled without it for the decks that need none, as that code's
 // register demand costs the move kernel ~5% in spills).
-// ROWSUM: see basis_lap_warp.
-template <typename Real, int MMAX, bool TB, int PER, bool XL = (MMAX <= 0), bool ROWSUM = false>
+// ROWSUM: see basis_lap_team.  TEAM: the walker's threads are a CtaTeam in the
+// local energy and the evaluation (moves and recomputes are one warp's work).
+template <typename Real, int MMAX, bool TB, int PER, bool XL = (MMAX <= 0), bool ROWSUM = false, bool TEAM = false>
 struct Walker {
   const DevSys<Real>& S;
   const WLayout& L;
@@ -55,6 +56,7 @@ struct Walker {
   unsigned char* sbase;  // scratch
   const Real* moc_s;     // [2][nbasis][mstride] MO coefficients (global, read through L1)
   int lane;
+  std::conditional_t<TEAM, CtaTeam, WarpTeam> tm;
   // MO column of the proposal from the tensor-core GEMM (tc_phase 2):
   // tcD[(row0 + q) * tc_ldd + i] = component q of orbital i
   const float* tcD = nullptr;
@@ -62,8 +64,12 @@ struct Walker {
   unsigned long long* ph = nullptr;  // phase counters (profiling builds)
   TBMove* tbm = nullptr;             // e-e-n tables of a proposal (TBX)
   // e-e-n terms from tables: the HBM-resident kernels but the fused step
-  // kernel, which keeps its arithmetic (basis_lap_warp)
+  // kernel, which keeps its arithmetic (basis_lap_team)
   static constexpr bool TBX = TB && MMAX <= 0 && !ROWSUM;
+  // the proposals in mixed precision only: the move kernel of a 128-electron
+  // cell (mixed, 1024 walkers) takes 46.1 ms with the tables and 49.5 without,
+  // that of a 32-electron cell 4.4 ms either way, in FP64 4.9 against 4.4
+  static constexpr bool TBXM = TBX && sizeof(Real) == 4;
   static constexpr bool CPX = MMAX < 0;
   // F and G basis shells and CUTOFF_MO: compiled into the HBM-resident kernels only
   static constexpr bool HL = MMAX < 0 || (MMAX == 0 && XL);
@@ -401,11 +407,12 @@ struct Walker {
     constexpr bool has3 = TB;
     NearSet nsn, nso;  // atoms in e-e-n range of the new and the old position
     bool tab = false;  // both in tbm with their radials
-    if constexpr (TBX) {
+    if constexpr (TBXM) {
       const double pn[3] = {px, py, pz}, po[3] = {ox, oy, oz};
-      tab = S.tb_tab && tb_move_tables(S, pn, po, *tbm, lane);
+      tab = tb_move_tables(S, pn, po, *tbm, lane);
     }
-    if (has3 && !tab) {
+    if (TBXM) nsn.n = nso.n = -1;  // without the tables: every atom
+    if constexpr (has3 && !TBXM) {
       const double pn[3] = {px, py, pz}, po[3] = {ox, oy, oz};
       near_atoms(S, pn, nsn);
       near_atoms(S, po, nso);
@@ -465,14 +472,14 @@ struct Walker {
       // gradient w.r.t. r_j of u(r_e - r_j) = -f'/r (r_e - r_j)
       double g0 = -fn * nx + fo * qx, g1 = -fn * ny + fo * qy, g2 = -fn * nz + fo * qz, l0 = ln - lo;
       if constexpr (has3) {
-        if (TBX && tab) {
+        if (TBXM && tab) {
           const double dn[3] = {nx, ny, nz}, dq[3] = {qx, qy, qz};
           const double rnd = sqrt(nx * nx + ny * ny + nz * nz), rqd = sqrt(qx * qx + qy * qy + qz * qz);
           double dgj[3] = {0, 0, 0}, dlj = 0;
           tb_pair_move_tab(S, *tbm, same, pj, dn, rnd, dq, rqd, du, ge, le, dgj, dlj);
           g0 += dgj[0]; g1 += dgj[1]; g2 += dgj[2];
           l0 += dlj;
-        } else if (nsn.n >= 0 && nso.n >= 0) {
+        } else if (!TBXM && nsn.n >= 0 && nso.n >= 0) {
           const double dn[3] = {nx, ny, nz}, dq[3] = {qx, qy, qz};
           const double rnd = sqrt(nx * nx + ny * ny + nz * nz), rqd = sqrt(qx * qx + qy * qy + qz * qz);
           double dgj[3] = {0, 0, 0}, dlj = 0;
@@ -495,11 +502,11 @@ struct Walker {
     }
     // one-body terms: lanes over (atom, function) pairs, those of the tables
     // where no function reaches beyond them
-    const bool obt = TBX && tab && S.ei_in_tb;
-    if constexpr (TBX) {
+    const bool obt = TBXM && tab && S.ei_in_tb;
+    if constexpr (TBXM) {
       const int n0 = obt ? tbm->n[0] : 0, n1 = obt ? tbm->n[1] : 0;
-      for (int idx = lane; idx < (n0 + n1) * QWG_TBK; idx += 32) {
-        const int el_ = idx / QWG_TBK, k = idx - el_ * QWG_TBK;
+      for (int idx = lane; idx < (n0 + n1) * S.en_k; idx += 32) {
+        const int el_ = idx / S.en_k, k = idx - el_ * S.en_k;
         const int side = el_ < n0 ? 0 : 1, q = side == 0 ? el_ : el_ - n0;
         const int t = S.atom_type[tbm->a[side][q]];
         if (k >= S.ei_n[t]) continue;
@@ -685,24 +692,24 @@ struct Walker {
   }
 
   // ---- local energy pieces
-  __device__ double kinetic() const {
+  __device__ double kinetic() {
     double k = 0;
-    for (int e = lane; e < S.nelec; e += 32) {
+    for (int e = tm.rank; e < S.nelec; e += tm.size()) {
       double g[3], l;
       electron_grad(e, g, l);
       k += l;
     }
-    return -0.5 * warp_sum(k);
+    return -0.5 * tm.sum(k);
   }
 
   // Periodic_system::ewaldElectron + the constant ion/self terms
   // (Periodic_system.cpp:586-973): real-space sums over the 27 images of the
   // minimum-image vectors, reciprocal sum over the kept G-vectors.
-  __device__ double ewald() const {
+  __device__ double ewald() {
     const double* Rp = R();
     const int N = S.nelec, A = S.natoms;
     double v = 0;
-    for (int idx = lane; idx < N * A; idx += 32) {
+    for (int idx = tm.rank; idx < N * A; idx += tm.size()) {
       const int e = idx / A, a = idx - e * A;
       double dx = Rp[3 * e] - S.atom_pos[a][0], dy = Rp[3 * e + 1] - S.atom_pos[a][1], dz = Rp[3 * e + 2] - S.atom_pos[a][2];
       min_image(S, dx, dy, dz);
@@ -714,7 +721,7 @@ struct Walker {
       }
       v -= S.atom_charge[a] * t;
     }
-    for (int idx = lane; idx < N * N; idx += 32) {
+    for (int idx = tm.rank; idx < N * N; idx += tm.size()) {
       const int i = idx / N, j = idx - i * N;
       if (i >= j) continue;
       double dx = Rp[3 * i] - Rp[3 * j], dy = Rp[3 * i + 1] - Rp[3 * j + 1], dz = Rp[3 * i + 2] - Rp[3 * j + 2];
@@ -725,7 +732,7 @@ struct Walker {
         v += erfc_poly(S.alpha * r) / r;
       }
     }
-    for (int g = lane; g < S.ng; g += 32) {
+    for (int g = tm.rank; g < S.ng; g += tm.size()) {
       const double* G = S.gvec + 3 * g;
       double ss = 0, cs = 0;
       for (int e = 0; e < N; e++) {
@@ -736,28 +743,28 @@ struct Walker {
       const double w = S.gweight[g];
       v += 2.0 * (-(S.ion_cos[g] * cs + S.ion_sin[g] * ss) * w + (cs * cs + ss * ss) * w / 2);
     }
-    return warp_sum(v) + S.ewald_const;
+    return tm.sum(v) + S.ewald_const;
   }
 
   // Molecular_system::calcLoc (Molecular_system.cpp:209-287), no field.
-  __device__ double coulomb() const {
+  __device__ double coulomb() {
     if (PER == 1 || (PER == 2 && S.periodic)) return ewald();
     const double* Rp = R();
     const int N = S.nelec, A = S.natoms;
     double v = 0;
-    for (int idx = lane; idx < N * A; idx += 32) {
+    for (int idx = tm.rank; idx < N * A; idx += tm.size()) {
       int e = idx / A, a = idx - e * A;
       const double* ap = S.atom_pos[a];
       double dx = Rp[3 * e] - ap[0], dy = Rp[3 * e + 1] - ap[1], dz = Rp[3 * e + 2] - ap[2];
       v -= S.atom_charge[a] / sqrt(dx * dx + dy * dy + dz * dz);
     }
-    for (int idx = lane; idx < N * N; idx += 32) {
+    for (int idx = tm.rank; idx < N * N; idx += tm.size()) {
       int i = idx / N, j = idx - i * N;
       if (i >= j) continue;
       double dx = Rp[3 * i] - Rp[3 * j], dy = Rp[3 * i + 1] - Rp[3 * j + 1], dz = Rp[3 * i + 2] - Rp[3 * j + 2];
       v += 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
     }
-    return warp_sum(v) + S.ion_ion;
+    return tm.sum(v) + S.ion_ion;
   }
 
   // Radial v_l(r) of channel l for an electron of spin s (SPIN_DEP tables
@@ -795,14 +802,14 @@ struct Walker {
     const int N = S.nelec, A = S.natoms;
     double vloc = 0;
     if (tmoves)
-      for (int e = lane; e < N; e += 32) moves[4 * e + 3] = 0.0;
+      for (int e = tm.rank; e < N; e += tm.size()) moves[4 * e + 3] = 0.0;
     double res_total = 1.0, res_x = 0, res_y = 0, res_z = 0;  // one-move-per-walker reservoir
     int res_e = -1;
     // per-electron Jastrow value at the current position
     QWG_PHASE_BEGIN(t_ue)
-    for (int e = TBX ? N : lane; e < N; e += 32)  // TBX: chunk by chunk below
+    for (int e = TBX ? N : tm.rank; e < N; e += tm.size())  // TBX: chunk by chunk below
       Ue()[e] = double(jas_electron_val<Real, TB>(S, Rp, e, Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2]));
-    __syncwarp();
+    tm.sync();
     QWG_PHASE_END(t_ue, PH_PP_JASTROW, ph)
     double vnl = 0;
     // electrons in chunks of L.wchunk: the (electron, atom) items of the
@@ -817,8 +824,8 @@ struct Walker {
     size_t en_at = 0;
     bool en_ok = false;
     if constexpr (TBX) {
-      const size_t end = sizeof(PPItem) * (size_t)CH * A, need = (size_t)N * (8 + (size_t)A * QWG_TBK * sizeof(Real));
-      if (S.tb_tab && need <= end) {
+      const size_t end = sizeof(PPItem) * (size_t)CH * A, need = (size_t)N * (8 + (size_t)A * S.en_k * sizeof(Real));
+      if (need <= end) {
         en_at = end - need;
         en.val = (Real*)((unsigned char*)it + en_at);
         en.near = (unsigned long long*)((unsigned char*)it + end - (size_t)N * 8);
@@ -828,8 +835,8 @@ struct Walker {
       const int e1 = min(N, e0 + CH);
       QWG_PHASE_BEGIN(t_items)
       int nitems = 0;
-      for (int base0 = e0 * A; base0 < e1 * A; base0 += 32) {
-        const int idx = base0 + lane;
+      for (int base0 = e0 * A; base0 < e1 * A; base0 += tm.size()) {
+        const int idx = base0 + tm.rank;
         bool take = false;
         PPItem item;
         if (idx < e1 * A) {
@@ -858,34 +865,34 @@ struct Walker {
             }
           }
         }
-        unsigned m = __ballot_sync(0xffffffffu, take);
-        int pos = nitems + __popc(m & ((1u << lane) - 1u));
+        int taken;
+        const int pos = nitems + tm.rank_among(take, taken);
         if (take) it[pos] = item;
-        nitems += __popc(m);
+        nitems += taken;
       }
-      __syncwarp();
+      tm.sync();
       QWG_PHASE_END(t_items, PH_PP_ITEMS, ph)
       if constexpr (TBX) {
         if (!en.val || nitems * sizeof(PPItem) > en_at) en_ok = false;
         else if (!en_ok && nitems > 0) {
-          en_table_fill(S, Rp, en, lane, 32);
-          en_table_near(S, Rp, en, lane, 32);
+          en_table_fill(S, Rp, en, tm.rank, tm.size());
+          en_table_near(S, Rp, en, tm.rank, tm.size());
           en_ok = true;
-          __syncwarp();
+          tm.sync();
         }
       }
       if (nitems == 0) continue;
       if constexpr (TBX) {
-        for (int e = e0 + lane; e < e1; e += 32) {
+        for (int e = e0 + tm.rank; e < e1; e += tm.size()) {
           const double* p = Rp + 3 * e;
           Ue()[e] = double(en_ok ? jas_point_val(S, Rp, e, p[0], p[1], p[2], en)
                                  : jas_electron_val<Real, TB>(S, Rp, e, p[0], p[1], p[2]));
         }
-        __syncwarp();
+        tm.sync();
       }
       QWG_PHASE_BEGIN(t_proj)
       const int nproj = multi() ? L.nud : 1;  // projected-coefficient sets per electron
-      for (int idx = lane; idx < (e1 - e0) * S.nbasis * nproj && multi(); idx += 32) {
+      for (int idx = tm.rank; idx < (e1 - e0) * S.nbasis * nproj && multi(); idx += tm.size()) {
         // one set per distinct spin-determinant u: w_f = sum_i C[f][col_u(i)] (A_u^-1)[i][e]
         const int u = idx / ((e1 - e0) * S.nbasis), r = idx - u * (e1 - e0) * S.nbasis;
         const int le = r / S.nbasis, f = r - le * S.nbasis;
@@ -898,7 +905,7 @@ struct Walker {
         for (int m = 0; m < M; m++) acc += cf[cu[m]] * iv[m];
         w[((size_t)u * CH + le) * S.nbasis + f] = acc;
       }
-      for (int idx = lane; idx < (e1 - e0) * S.nbasis && CPX; idx += 32) {
+      for (int idx = tm.rank; idx < (e1 - e0) * S.nbasis && CPX; idx += tm.size()) {
         // complex w_f = sum_m C[f][m] invT[el][m]
         const int le = idx / S.nbasis, f = idx - le * S.nbasis;
         const int e = e0 + le, s = spin(e), el = eloc(e), M = S.m[s];
@@ -914,28 +921,31 @@ struct Walker {
         w[le * S.nbasis + f] = ar;
         w[wproj_im_off() + le * S.nbasis + f] = ai;
       }
-      for (int idx = lane; idx < (e1 - e0) * S.nbasis && !multi() && !CPX; idx += 32) {
+      for (int idx = tm.rank; idx < (e1 - e0) * S.nbasis && !multi() && !CPX; idx += tm.size()) {
         const int le = idx / S.nbasis, f = idx - le * S.nbasis;
         const int e = e0 + le, s = spin(e), el = eloc(e), M = S.m[s];
-        const Real* cf = mocs(s) + (size_t)f * MS();
         const Real* iv = inv(s) + (size_t)el * MS();
         Real acc = Real(0);
         if constexpr (MMAX > 0) {
+          const Real* cf = mocs(s) + (size_t)f * MS();
 #pragma unroll
           for (int m = 0; m < MMAX; m++)
             if (m < M) acc += cf[m] * iv[m];
         } else {
-          for (int m = 0; m < M; m++) acc += cf[m] * iv[m];
+          // lanes over the basis functions: a row of the transposed
+          // coefficients is one line of memory per orbital, not one per lane
+          const Real* cf = S.moct + (size_t)s * MS() * S.nbasis + f;
+          for (int m = 0; m < M; m++) acc += cf[(size_t)m * S.nbasis] * iv[m];
         }
         w[le * S.nbasis + f] = acc;
       }
-      __syncwarp();
+      tm.sync();
       QWG_PHASE_END(t_proj, PH_PP_PROJECT, ph)
       QWG_PHASE_BEGIN(t_pts)
       int total = 0;
       for (int k = 0; k < nitems; k++) total += S.pp_aip[S.atom_type[it[k].a]];
       int k = 0, qoff = 0;  // running item cursor for this lane's points
-      for (int p = lane; p < total; p += 32) {
+      for (int p = tm.rank; p < total; p += tm.size()) {
         while (p >= qoff + S.pp_aip[S.atom_type[it[k].a]]) { qoff += S.pp_aip[S.atom_type[it[k].a]]; k++; }
         const PPItem& I = it[k];
         const int q = p - qoff;
@@ -996,7 +1006,7 @@ struct Walker {
         vnl += ts * ratio;
         if (tmoves) cand[p] = ts * ratio;
       }
-      __syncwarp();
+      tm.sync();
       QWG_PHASE_END(t_pts, PH_PP_POINTS, ph)
       if (tmoves) {
         // target of point p of this chunk (the same arithmetic as above)
@@ -1014,7 +1024,7 @@ struct Walker {
         if (tmoves == 2) {
           // size-consistent: lanes over the chunk's electrons; the points of
           // one electron are contiguous (items are in electron order)
-          for (int e = e0 + lane; e < e1; e += 32) {
+          for (int e = e0 + tm.rank; e < e1; e += tm.size()) {
             int pb = 0, k = 0;
             for (; k < nitems && it[k].e < e; k++) pb += S.pp_aip[S.atom_type[it[k].a]];
             int pe = pb;
@@ -1062,15 +1072,15 @@ struct Walker {
             }
           }
         }
-        __syncwarp();
+        tm.sync();
       }
     }
-    if (tmoves == 1 && res_e >= 0 && lane == 0) {
+    if (tmoves == 1 && res_e >= 0 && tm.rank == 0) {
       moves[4 * res_e] = res_x; moves[4 * res_e + 1] = res_y; moves[4 * res_e + 2] = res_z;
       moves[4 * res_e + 3] = 1.0;
     }
-    __syncwarp();
-    return warp_sum(vloc) + warp_sum(vnl);
+    tm.sync();
+    return tm.sum(vloc) + tm.sum(vnl);
   }
 };
 
@@ -1122,8 +1132,12 @@ template <typename Real, int MMAX, int mode, bool TB, int PER, bool XL = (MMAX <
 __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
     k_walkers(const __grid_constant__ DevSys<Real> S, const __grid_constant__ WLayout L, StepParams P, EvalIO io) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int wpc = blockDim.x / 32;
-  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  constexpr bool HBM = MMAX <= 0;  // walker worked on in place in HBM
+  constexpr bool TEAM = HBM && (mode == KM_EVAL || mode == KM_ELOC || mode == KM_ELOC_TM || mode == KM_SWEEP);
+  const int lane = threadIdx.x & 31;
+  const int tsize = TEAM ? 32 * P.team : 32;  // threads per walker
+  const int wpc = blockDim.x / tsize;
+  const int warp = threadIdx.x / tsize;       // walker of the CTA
   // MO coefficients are read through L1 (a few kB shared by every walker);
   // shared memory holds walker state only
   const Real* moc_s = S.moc;
@@ -1133,14 +1147,20 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
   __syncthreads();
 
   const int wid = blockIdx.x * wpc + warp;
-  constexpr bool HBM = MMAX <= 0;  // walker worked on in place in HBM
   constexpr bool CPXK = MMAX < 0;  // complex orbitals
   if (wid < P.nwalk) {
     unsigned char* gstate = P.state + (size_t)wid * L.state_bytes;
     constexpr bool SWEEP_ONLY = mode == KM_SWEEP || mode == KM_TMOVE;  // move-phase shared memory only
     unsigned char* wb = HBM ? gstate : smem + moc_bytes + (size_t)warp * (SWEEP_ONLY ? L.sweep_bytes : L.bytes);
     unsigned char* sb = HBM ? P.scratch + (size_t)wid * L.scratch_bytes : wb + L.state_bytes;
-    Walker<Real, MMAX, TB, PER, XL, mode == KM_STEPS> W{S, L, wb, sb, moc_s, lane};
+    Walker<Real, MMAX, TB, PER, XL, mode == KM_STEPS, TEAM> W{S, L, wb, sb, moc_s, lane, {}};
+    auto& tm = W.tm;
+    if constexpr (TEAM) {
+      __shared__ double exchange[4 * TEAM_SLOT];
+      tm = CtaTeam{(int)threadIdx.x - warp * tsize, tsize, 1 + warp, 0, exchange + warp * TEAM_SLOT};
+    } else {
+      tm.rank = lane;
+    }
     if constexpr (TB && HBM && (mode == KM_SWEEP || mode == KM_RATIO || mode == KM_TMOVE)) {
       __shared__ TBMove tables[4];
       W.tbm = tables + warp;
@@ -1166,6 +1186,7 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
     if (tc_phase == 2 || (tc_phase == 1 && P.tc_e > 0)) refresh = 0;  // the sweep's first launch only
     constexpr bool STEPS = mode == KM_STEPS || mode == KM_SWEEP || ELOCM || mode == KM_TMOVE;
     if (!STEPS || refresh) {
+     if (tm.warp() == 0) {  // one warp's work
       for (int i = lane; i < 3 * N; i += 32) Rp[i] = P.R[(size_t)wid * 3 * N + i];
       __syncwarp();
       if (S.periodic)
@@ -1178,6 +1199,8 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
       QWG_PHASE_END(t_ref, PH_REFRESH, P.phases)
       if (lane == 0 && STEPS) { W.sc()->eold = keep_e; W.sc()->weight = keep_w; }
       __syncwarp();
+     }
+      tm.sync();
     } else if constexpr (!HBM) {
       // resident state: one coalesced copy HBM -> shared memory
       const int4* src = (const int4*)gstate;
@@ -1190,7 +1213,7 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
       double rm[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
       if (io.rot)
         for (int k = 0; k < 9; k++) rm[k] = io.rot[(size_t)wid * 9 + k];
-      for (int e = lane; e < N; e += 32) {
+      for (int e = tm.rank; e < N; e += tm.size()) {
         double g[3], l;
         W.electron_grad(e, g, l);
         double* go = io.grad + ((size_t)wid * N + e) * 3;
@@ -1208,7 +1231,7 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
         else
           nl = W.pseudo(rm, true, 0, wid, 0);
       }
-      if (lane == 0) {
+      if (tm.rank == 0) {
         WScal* w = W.sc();
         if (W.multi()) {
           double sgn;
@@ -1313,17 +1336,18 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
               // basis rows of the proposed position -> split-TF32 A rows of
               // this walker (rows wid * 5 + component)
               Real* b = W.bas();
-              basis_lap_warp<Real, PER, (MMAX < 0 || (MMAX == 0 && XL))>(S, wx, wy, wz, b, lane);
+              basis_lap_team<Real, PER, (MMAX < 0 || (MMAX == 0 && XL))>(S, wx, wy, wz, b, tm);
               float* ah = P.tc_ahi + (size_t)wid * 5 * P.tc_kpad;
               float* al = P.tc_alo + (size_t)wid * 5 * P.tc_kpad;
-              for (int idx = lane; idx < 5 * P.tc_kpad; idx += 32) {
-                const int c = idx / P.tc_kpad, f = idx - c * P.tc_kpad;
-                const float v = f < S.nbasis ? float(b[(size_t)f * 5 + c]) : 0.0f;
-                float hi, lo;
-                tc_split_tf32(v, hi, lo);
-                ah[idx] = hi;
-                al[idx] = lo;
-              }
+              for (int f = tm.rank; f < P.tc_kpad; f += tm.size())
+#pragma unroll
+                for (int c = 0; c < 5; c++) {
+                  const float v = f < S.nbasis ? float(b[(size_t)f * 5 + c]) : 0.0f;
+                  float hi, lo;
+                  tc_split_tf32(v, hi, lo);
+                  ah[c * P.tc_kpad + f] = hi;
+                  al[c * P.tc_kpad + f] = lo;
+                }
               continue;
             }
             double ratioD, dU, g1[3], l1;
@@ -1434,12 +1458,12 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
             wt = w->weight * exp(teffac * (etr * 2 - el - eold));
             if (wt > P.max_weight) wt = P.max_weight;
             if (!isfinite(el) || !isfinite(wt)) { nbad += 1; wt = 0.0; el = etr; }
-            __syncwarp();
-            if (lane == 0) { w->weight = wt; w->eold = el; }
-            __syncwarp();
+            tm.sync();
+            if (tm.rank == 0) { w->weight = wt; w->eold = el; }
+            tm.sync();
           } else {
             if (!isfinite(el)) { nbad += 1; el = 0.0; wt = 0.0; }
-            if (lane == 0) w->eold = el;
+            if (tm.rank == 0) w->eold = el;
           }
           sw += wt; swe += wt * el; swk += wt * kin; swv += wt * pot; swnl += wt * nl; swe2 += wt * el * el;
           u[0] += el; u[1] += el * el; u[2] += kin; u[3] += kin * kin; u[4] += pot; u[5] += pot * pot;
@@ -1448,7 +1472,7 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
         }
       }
       QWG_PHASE_END(t_walker, PH_WALKER, P.phases)
-      if (lane == 0) {
+      if (tm.rank == 0) {
         if (!ELOCM) { atomicAdd(&cta_acc[6], nacc); atomicAdd(&cta_acc[7], natt); }
         if (mode != KM_SWEEP) {
           atomicAdd(&cta_acc[0], sw); atomicAdd(&cta_acc[1], swe); atomicAdd(&cta_acc[2], swk);
@@ -1461,16 +1485,16 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
       }
       // write back: positions and the resident state after moves; only the
       // walker scalars after a local-energy pass
-      __syncwarp();
+      tm.sync();
       if (!ELOCM)
-        for (int i = lane; i < 3 * N; i += 32) P.R[(size_t)wid * 3 * N + i] = Rp[i];
+        for (int i = tm.rank; i < 3 * N; i += tm.size()) P.R[(size_t)wid * 3 * N + i] = Rp[i];
       if constexpr (!HBM) {
         int4* dst = (int4*)gstate;
         const int4* src = (const int4*)wb;
         if (ELOCM) {
-          for (int i = lane; i < (int)sizeof(WScal) / 16; i += 32) ((int4*)(gstate + L.scal))[i] = ((const int4*)(wb + L.scal))[i];
+          for (int i = tm.rank; i < (int)sizeof(WScal) / 16; i += tm.size()) ((int4*)(gstate + L.scal))[i] = ((const int4*)(wb + L.scal))[i];
         } else {
-          for (int i = lane; i < L.state_bytes / 16; i += 32) dst[i] = src[i];
+          for (int i = tm.rank; i < L.state_bytes / 16; i += tm.size()) dst[i] = src[i];
         }
       }
     }

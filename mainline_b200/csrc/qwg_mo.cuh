@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(128) k_basis_rows_tf32(const __grid_constant__
   double x = pos[3 * p], y = pos[3 * p + 1], z = pos[3 * p + 2];
   if (S.periodic) wrap_pos(S, x, y, z);
   double* bas = bas_scratch + (size_t)p * S.nbasis * 5;
-  basis_lap_warp<double, 2, true>(S, x, y, z, bas, lane);
+  basis_lap_team<double, 2, true>(S, x, y, z, bas, WarpTeam{lane});
   for (int idx = lane; idx < 5 * kpad; idx += 32) {
     const int c = idx / kpad, f = idx - c * kpad;
     const double v = f < S.nbasis ? bas[(size_t)f * 5 + c] : 0.0;

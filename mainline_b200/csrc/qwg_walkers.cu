@@ -1,5 +1,6 @@
 // One walker-kernel family: compiled once per (QWG_REAL, QWG_MM) pair by the
 // build (e.g. -DQWG_REAL=float -DQWG_MM=32).
+#include <algorithm>
 #include <map>
 #include <mutex>
 
@@ -51,8 +52,10 @@ cudaError_t launch_mode(const DevSys<Real>& S, const WLayout& L, const StepParam
   cudaError_t e = ensure_smem_attr(kern, smem);
   if (e != cudaSuccess) return e;
   if (nwalk <= 0) return cudaSuccess;  // attribute set only (before a stream capture)
-  const int grid = (nwalk + wpc - 1) / wpc;
-  kern<<<grid, 32 * wpc, smem, stream>>>(S, L, P, io);
+  // HBM-resident walkers: P.team warps each, at most 4 warps per CTA
+  const int team = MM <= 0 ? P.team : 1, per = MM <= 0 ? std::max(1, std::min(wpc, 4 / team)) : wpc;
+  const int grid = (nwalk + per - 1) / per;
+  kern<<<grid, 32 * team * per, smem, stream>>>(S, L, P, io);
   return cudaGetLastError();
 }
 
