@@ -120,7 +120,7 @@ struct qwg_ctx {
   long long launches = 0;
   // tables
   DevBuf d_moct;  // MO coefficients, a row per orbital (HBM-resident kernels)
-  DevBuf d_shell_i, d_shell_obj, d_shell_cut, d_shell_order, d_spline, d_spline64, d_moc, d_moc_im, d_image_kfac;
+  DevBuf d_shell_i, d_shell_obj, d_shell_cut, d_row_cut, d_spline, d_spline64, d_moc, d_moc_im, d_image_kfac;
   DevBuf d_image_pos, d_gvec, d_gweight, d_ion_sin, d_ion_cos;
   DevBuf d_sub_seg, d_sub_idx;  // sub-cell candidate lists of the image sums
   int sub_n[3] = {0, 0, 0};
@@ -207,7 +207,7 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
   S.shell_i = c->d_shell_i.as<int4>();
   S.shell_obj = c->d_shell_obj.as<int2>();
   S.shell_cut = c->d_shell_cut.as<double>();
-  S.shell_order = c->d_shell_order.as<int>();
+  S.row_cut = c->d_row_cut.as<double>();
   S.spline = c->d_spline.as<Real>();
   S.spline64 = c->d_spline64.as<double>();
   S.moc = c->d_moc.as<Real>();
@@ -455,22 +455,26 @@ static void build_tables(qwg_ctx* c) {
               H.spline_coef[((size_t)(H.obj_first[o] + k) * npts + i) * 4 + q];
   std::vector<int4> si;
   std::vector<int2> so;
-  std::vector<double> sc;
-  for (size_t k = 0; k < H.shells.size(); k++) {
-    const Shell& s = H.shells[k];
-    si.push_back(make_int4(s.center, s.sym, s.first, s.k));
-    so.push_back(make_int2(obj_base[s.obj], H.obj_count[s.obj]));
-    sc.push_back(H.cutoff_mo ? s.fcut : s.cutoff);  // CUTOFF_MO: each function inside its own cutoff
+  std::vector<double> sc, rc;
+  // CUTOFF_MO: each function inside its own cutoff
+  const auto cutoff = [&](const Shell& s) { return H.cutoff_mo ? s.fcut : s.cutoff; };
+  std::vector<const Shell*> order;  // by shape, the longest first
+  for (const Shell& s : H.shells) {
+    sc.push_back(cutoff(s));
+    order.push_back(&s);
+  }
+  if (order.size() > 32)  // one round of a warp takes the shells in any order
+    std::stable_sort(order.begin(), order.end(), [](const Shell* a, const Shell* b) { return a->sym > b->sym; });
+  for (const Shell* s : order) {
+    si.push_back(make_int4(s->center, s->sym, s->first, s->k));
+    so.push_back(make_int2(obj_base[s->obj], H.obj_count[s->obj]));
+    rc.push_back(cutoff(*s));
   }
   (void)A;
   upload(c->d_shell_i, si, st);
   upload(c->d_shell_obj, so, st);
   upload(c->d_shell_cut, sc, st);
-  // image sums: the shells by shape
-  std::vector<int> order(H.shells.size());
-  for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return H.shells[a].sym > H.shells[b].sym; });
-  upload(c->d_shell_order, order, st);
+  upload(c->d_row_cut, rc, st);
   // MO coefficients padded to the orbital stride, both spins
   const int mm = mo_stride_for(c->mmax, std::max(H.nmo[0], H.nmo[1]));
   std::vector<double> moc((size_t)2 * H.nbasis * mm, 0.0), moc_im(moc.size(), 0.0);
@@ -695,7 +699,7 @@ static size_t footprint_bytes(const qwg_ctx* c, int max_walkers) {
   size_t total4 = 0;
   for (size_t o = 0; o < H.obj_first.size(); o++) total4 += (size_t)H.spline_npts * H.obj_count[o];
   const size_t ms = mo_stride_for(c->mmax, std::max(H.nmo[0], H.nmo[1]));
-  size_t b = total4 * 4 * (8 + rs) + 2 * (size_t)H.nbasis * ms * rs * (hbm_family(c->mmax) ? 2 : 1) + H.shells.size() * 36 +
+  size_t b = total4 * 4 * (8 + rs) + 2 * (size_t)H.nbasis * ms * rs * (hbm_family(c->mmax) ? 2 : 1) + H.shells.size() * 40 +
              H.image_pos.size() * 8 * 5 / 3 + H.gvec.size() * 8 + 3 * H.gweight.size() * 8;
   if (H.periodic) {
     const SubcellLists sl = make_subcell_lists(H);

@@ -36,6 +36,10 @@ struct PPItem {
   double vl[4];          // nonlocal channel radials (already scaled)
 };
 
+// Four consecutive elements of a row that starts on 16 bytes.
+template <typename Real>
+struct alignas(16) Quad { Real x[4]; };
+
 // MMAX > 0: at most MMAX orbitals per spin, state + scratch in shared
 // memory.  MMAX == 0: any count up to 256 per spin, arrays strided by
 // L.mstride and worked on in place in HBM.  MMAX == -1 (QWG_MM_CPX): the
@@ -46,7 +50,8 @@ struct PPItem {
 // XL: the F/G-shell and CUTOFF_MO code (HBM-resident kernels; the FP32 ones
 // are also compiled without it for the decks that need none, as that code's
 // register demand costs the move kernel ~5% in spills).
-// ROWSUM: see basis_lap_team.  TEAM: the walker's threads are a CtaTeam in the
+// ROWSUM: see basis_lap_team (the shared-memory kernels always, which only a
+// deck forced onto them brings a periodic cell).  TEAM: the walker's threads are a CtaTeam in the
 // local energy and the evaluation (moves and recomputes are one warp's work).
 template <typename Real, int MMAX, bool TB, int PER, bool XL = (MMAX <= 0), bool ROWSUM = false, bool TEAM = false>
 struct Walker {
@@ -399,8 +404,15 @@ struct Walker {
     }
     QWG_PHASE_BEGIN(t_rest)
     ratioD = double(r0);
-    double gD[3] = {double(r1) / ratioD, double(r2) / ratioD, double(r3) / ratioD};
-    double lD = double(r4) / ratioD;
+    double gD[3], lD;
+    if constexpr (ROWSUM || sizeof(Real) == 8) {
+      gD[0] = double(r1) / ratioD; gD[1] = double(r2) / ratioD; gD[2] = double(r3) / ratioD;
+      lD = double(r4) / ratioD;
+    } else {
+      const double ir = 1.0 / ratioD;  // one quotient for four
+      gD[0] = r1 * ir; gD[1] = r2 * ir; gD[2] = r3 * ir;
+      lD = r4 * ir;
+    }
     // Jastrow: lanes over the other electrons
     const double ox = Rp[3 * e], oy = Rp[3 * e + 1], oz = Rp[3 * e + 2];
     const bool se = s == 0;
@@ -648,7 +660,16 @@ struct Walker {
     }
     __syncwarp();
     const Real invr = Real(1.0 / ratioD);
-    for (int idx = lane; idx < M * M && !multi() && !CPX; idx += 32) {
+    if constexpr (MMAX == 8) {
+      // rows of 8: no index division
+      for (int idx = lane; idx < 8 * M; idx += 32) {
+        const int k = idx >> 3, i = idx & 7;
+        if (i >= M) continue;
+        if (k == el) iv[idx] = rowe[i] * invr;
+        else iv[idx] -= rowe[i] * wk[k] * invr;
+      }
+    }
+    for (int idx = lane; idx < M * M && MMAX != 8 && !multi() && !CPX; idx += 32) {
       int k = idx / M, i = idx - k * M;
       if (k == el) iv[(size_t)k * ms + i] = rowe[i] * invr;
       else iv[(size_t)k * ms + i] -= rowe[i] * wk[k] * invr;
@@ -927,10 +948,26 @@ struct Walker {
         const Real* iv = inv(s) + (size_t)el * MS();
         Real acc = Real(0);
         if constexpr (MMAX > 0) {
-          const Real* cf = mocs(s) + (size_t)f * MS();
+          const Real* row = mocs(s) + (size_t)f * MS();
+          if (sizeof(Real) == 4 && M > 4) {
+            // rows padded to MMAX: four elements a load (local energy of the
+            // two-atom molecule, mixed: 0.300 -> 0.285 ms; in FP64 and for at
+            // most 4 orbitals up to 2% slower than one by one)
+            const Quad<Real>* cf = reinterpret_cast<const Quad<Real>*>(row);
+            const Quad<Real>* iq = reinterpret_cast<const Quad<Real>*>(iv);
 #pragma unroll
-          for (int m = 0; m < MMAX; m++)
-            if (m < M) acc += cf[m] * iv[m];
+            for (int m = 0; m < MMAX; m += 4) {
+              if (m >= M) break;
+              const Quad<Real> a = cf[m / 4], b = iq[m / 4];
+#pragma unroll
+              for (int q = 0; q < 4; q++)
+                if (m + q < M) acc += a.x[q] * b.x[q];
+            }
+          } else {
+#pragma unroll
+            for (int m = 0; m < MMAX; m++)
+              if (m < M) acc += row[m] * iv[m];
+          }
         } else {
           // lanes over the basis functions: a row of the transposed
           // coefficients is one line of memory per orbital, not one per lane
@@ -1153,7 +1190,7 @@ __global__ void __launch_bounds__(128, MinBlocks<mode>::value)
     constexpr bool SWEEP_ONLY = mode == KM_SWEEP || mode == KM_TMOVE;  // move-phase shared memory only
     unsigned char* wb = HBM ? gstate : smem + moc_bytes + (size_t)warp * (SWEEP_ONLY ? L.sweep_bytes : L.bytes);
     unsigned char* sb = HBM ? P.scratch + (size_t)wid * L.scratch_bytes : wb + L.state_bytes;
-    Walker<Real, MMAX, TB, PER, XL, mode == KM_STEPS, TEAM> W{S, L, wb, sb, moc_s, lane, {}};
+    Walker<Real, MMAX, TB, PER, XL, !HBM || mode == KM_STEPS, TEAM> W{S, L, wb, sb, moc_s, lane, {}};
     auto& tm = W.tm;
     if constexpr (TEAM) {
       __shared__ double exchange[4 * TEAM_SLOT];
