@@ -98,6 +98,7 @@ struct DevSys {
   int atom_type[QWG_MAXA];
   int4 center_seg[QWG_MAXA];     // (first shell, shells, spline-object base, splines in the object)
   double center_cut[QWG_MAXA];   // basis-object threshold of the center
+  int center_first[QWG_MAXA];    // first basis function of the center
   // image sums on BLAS_MO: (S shells, P shells) of a center that has no
   // others, its shell_pack entries in that order; (0, 0) for other centers
   int2 center_sp[QWG_MAXA];
@@ -1254,7 +1255,7 @@ __device__ __forceinline__ Real basis_dot_lane_periodic(const DevSys<Real>& S, d
     int nfa = 0;
     for (int k = 0; k < cs.y; k++) nfa += sym_nfunc(S.shell_pack[cs.x + k] & 0xf);
     for (int q = 0; q < QWG_MAXF_ATOM; q++) fs[q] = Real(0);
-    const int fb0 = (S.shell_pack[cs.x] >> 4) & 0xffff;
+    const int fb0 = S.center_first[c];  // not the first entry's: center_sp centers list S before P
     const ImgRange im = images_of(S, sc, c);
     const Real cut = Real(S.center_cut[c]);
     const Real cut2 = cut * cut * Real(1.000001);  // beyond it rd < cut is certainly false

@@ -247,6 +247,7 @@ static void fill_sys(qwg_ctx* c, DevSys<Real>& S, const std::vector<int>& obj_ba
       seen[sh.center] = 1;
       cs = make_int4((int)k, 0, obj_base[sh.obj], H.obj_count[sh.obj]);
       S.center_cut[sh.center] = sh.cutoff;
+      S.center_first[sh.center] = sh.first;
     } else if (obj_base[sh.obj] != cs.z) {
       throw InputError("one BASIS section per atom label is supported");
     }
