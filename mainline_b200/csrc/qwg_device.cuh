@@ -509,8 +509,10 @@ struct CtaTeam {
   __device__ __forceinline__ int size() const { return n; }
   __device__ __forceinline__ int warp() const { return rank >> 5; }
   __device__ __forceinline__ void sync() const {
-    if (n == 32) __syncwarp();
-    else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory");
+    // callers arrive from divergent loops: the barrier is the form that counts
+    // threads and needs no converged warp (the aligned one is undefined there)
+    __syncwarp();
+    if (n > 32) __barrier_sync_count(bar, n);
   }
   __device__ __forceinline__ double sum(double v) {
     v = warp_sum(v);
