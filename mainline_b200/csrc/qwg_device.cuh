@@ -82,7 +82,6 @@ struct DevSys {
   const int4* shell_i;           // (center, sym, first, k)
   const int2* shell_obj;         // (table base in 4-tuples, splines in the object)
   const double* shell_cut;       // [nshell], in the order of shell_pack
-  const double* row_cut;         // [nshell] shell_cut in the order of shell_i
   // radial spline tables, interval-major per basis object: the 4 cubic
   // coefficients of every spline of an object for interval i are contiguous
   // (one row of nk x 4 values), so all shells of a center read one row.
@@ -91,17 +90,12 @@ struct DevSys {
   int npts;
   double spacing, inv_spacing;
   const Real* moc;               // [2][nbasis][mstride]
-  const Real* moct;              // [2][mstride][nbasis] (HBM-resident real kernels)
   // ---- parameter-bank tables
   double atom_pos[QWG_MAXA][3];
   double atom_charge[QWG_MAXA];
   int atom_type[QWG_MAXA];
   int4 center_seg[QWG_MAXA];     // (first shell, shells, spline-object base, splines in the object)
   double center_cut[QWG_MAXA];   // basis-object threshold of the center
-  int center_first[QWG_MAXA];    // first basis function of the center
-  // image sums on BLAS_MO: (S shells, P shells) of a center that has no
-  // others, its shell_pack entries in that order; (0, 0) for other centers
-  int2 center_sp[QWG_MAXA];
   int shell_pack[QWG_MAXSHELL];  // sym | first << 4 | k << 20
   // Jastrow
   int nee;
@@ -112,9 +106,6 @@ struct DevSys {
   double onebody[QWG_MAXT][QWG_MAXEI];
   int tb_n[QWG_MAXT];
   double tb_rc[QWG_MAXT];        // largest e-i cutoff the type's e-e-n terms use
-  int tb_ee[QWG_MAXT];           // e-e functions the type's e-e-n terms use (bit mask)
-  int ei_in_tb;                  // every e-i function vanishes beyond its type's tb_rc
-  double ei_rc2[QWG_MAXT];       // (largest e-i cutoff of the type)^2 (1 + 1e-6)
   double ee_rc2;                 // (largest e-e cutoff)^2 (1 + 1e-12): every pair term (two- and
                                  // three-body) vanishes for electrons at least that far apart
   DTB tb[QWG_MAXT][QWG_MAXTB];
@@ -125,7 +116,6 @@ struct DevSys {
   // saved e-n basis only when a group has a plain THREEBODY term, so with
   // THREEBODY_SPIN alone its quadrature ratios see the stale values.
   int tb_stale_ei;
-  int en_k;                      // largest ei_n: stride of the e-n tables
   // pseudopotential per type (nchan 0: none)
   int has_pp;
   int pp_nchan[QWG_MAXT], pp_aip[QWG_MAXT];
@@ -172,6 +162,19 @@ struct DevSys {
   const double* gweight;         // [ng]
   const double* ion_sin;         // [ng]
   const double* ion_cos;         // [ng]
+  // ---- tables of the HBM-resident kernels.  They stand last: the tables
+  // above are read through the constant cache by every kernel, and moving
+  // them apart costs the shared-memory kernels of small molecules up to 4%.
+  const Real* moct;              // [2][mstride][nbasis] (real orbitals)
+  const double* row_cut;         // [nshell] shell_cut in the order of shell_i
+  int center_first[QWG_MAXA];    // first basis function of the center
+  // image sums on BLAS_MO: (S shells, P shells) of a center that has no
+  // others, its shell_pack entries in that order; (0, 0) for other centers
+  int2 center_sp[QWG_MAXA];
+  int tb_ee[QWG_MAXT];           // e-e functions the type's e-e-n terms use (bit mask)
+  double ei_rc2[QWG_MAXT];       // (largest e-i cutoff of the type)^2 (1 + 1e-6)
+  int ei_in_tb;                  // every e-i function vanishes beyond its type's tb_rc
+  int en_k;                      // largest ei_n: stride of the e-n tables
 };
 
 // Minimum-image vector (Periodic_sample::minimum_image,
@@ -362,7 +365,6 @@ enum QwgPhase {
 
 struct StepParams {
   int nwalk;
-  int team;             // warps per walker (HBM-resident kernels): 1, 2 or 4
   int nsteps;
   int st;               // KM_SWEEP / KM_ELOC: step of the chunk this launch performs
   int refresh;          // 1: full recompute at start, 0: load state, 2: recompute when the
@@ -404,6 +406,7 @@ struct StepParams {
   float* tc_alo;
   const float* tc_D;
   unsigned long long* phases;  // [PH_COUNT] counters (profiling builds), or null
+  int team;             // warps per walker (HBM-resident kernels): 1, 2 or 4
 };
 
 // ---------------------------------------------------------------------------
