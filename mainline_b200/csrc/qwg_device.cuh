@@ -910,6 +910,19 @@ __device__ void basis_lap_images(const DevSys<Real>& S, double px, double py, do
   }
 }
 
+// x^2 + y^2 + z^2 with the roundings spelled out: left to the compiler, which
+// square is fused into the sum depends on the code around it, and a VMC walk
+// of 128 electrons grows that last bit to 1e-8 bohr in three steps.
+// 0: the compiler's choice.  1: x^2 + y^2 rounded each, z^2 fused (the
+// recomputes of the fused step kernel with e-e-n terms).  2: every square
+// rounded (its proposals).
+template <int SQ>
+__device__ __forceinline__ double sum_squares(double x, double y, double z) {
+  if constexpr (SQ == 0) return x * x + y * y + z * z;
+  const double xy = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
+  return SQ == 1 ? __fma_rn(z, z, xy) : __dadd_rn(xy, __dmul_rn(z, z));
+}
+
 // Basis value, gradient and Laplacian of every basis function at one
 // position, by the whole team: its threads split the shells (radial spline and
 // angular factors in FP64: the Laplacian of the tight shells cancels
@@ -919,7 +932,8 @@ __device__ void basis_lap_images(const DevSys<Real>& S, double px, double py, do
 // ROWSUM: image sums in the rows themselves, the code of the fused step
 // kernel: a VMC walk doubles a difference of one rounding every few moves, so
 // its kernel keeps the arithmetic, and runs keep their walks bit for bit.
-template <typename O, int PER, bool HL, bool ROWSUM = false, typename Real, class TM>
+// SQ: the rounding of the squared distances there (sum_squares).
+template <typename O, int PER, bool HL, bool ROWSUM = false, int SQ = 0, typename Real, class TM>
 __device__ void basis_lap_team(const DevSys<Real>& S, double px, double py, double pz, O* bas, const TM& tm) {
   if constexpr (!ROWSUM && PER != 0) {
     if (PER == 1 || S.periodic) {
@@ -972,7 +986,7 @@ __device__ void basis_lap_team(const DevSys<Real>& S, double px, double py, doub
       for (int t = 0; t < im.count; t++) {
         const double* cp = S.image_pos + 3 * im[t];
         double dx = px - cp[0], dy = py - cp[1], dz = pz - cp[2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
+        const double r2 = sum_squares<SQ>(dx, dy, dz);
         if (!(r2 < cut2)) continue;
         double r = sqrt(r2);
         if (!(r < cut)) continue;
@@ -999,10 +1013,10 @@ __device__ void basis_lap_team(const DevSys<Real>& S, double px, double py, doub
 // basis rows (basis_lap_team) in bas [nbasis][5] as Real, then lanes split
 // the (MO, component) outputs of the contraction with the MO coefficients
 // moc_s [nbasis][mstride].
-template <typename Real, int PER, bool HL = false, bool ROWSUM = false>
+template <typename Real, int PER, bool HL = false, bool ROWSUM = false, int SQ = 0>
 __device__ void mo_lap_warp(const DevSys<Real>& S, const Real* moc_s, double px, double py, double pz, int M,
                             Real* bas, Real* out, int lane) {
-  basis_lap_team<Real, PER, HL, ROWSUM>(S, px, py, pz, bas, WarpTeam{lane});
+  basis_lap_team<Real, PER, HL, ROWSUM, SQ>(S, px, py, pz, bas, WarpTeam{lane});
   __syncwarp();
   if (M > 32) {
     // many orbitals: lanes over MOs (coalesced coefficient rows), the basis

@@ -71,6 +71,8 @@ struct Walker {
   // e-e-n terms from tables: the HBM-resident kernels but the fused step
   // kernel, which keeps its arithmetic (basis_lap_team)
   static constexpr bool TBX = TB && MMAX <= 0 && !ROWSUM;
+  // squared distances of the basis rows in a recompute and in a proposal (sum_squares)
+  static constexpr int SQ_RECOMPUTE = TB && MMAX == 0 && ROWSUM ? 1 : 0, SQ_PROPOSE = 2 * SQ_RECOMPUTE;
   // the proposals in mixed precision only: the move kernel of a 128-electron
   // cell (mixed, 1024 walkers) takes 46.1 ms with the tables and 49.5 without,
   // that of a 32-electron cell 4.4 ms either way, in FP64 4.9 against 4.4
@@ -211,7 +213,7 @@ struct Walker {
       double* vals = mdv();
       for (int el = 0; el < M; el++) {
         const int e = e0 + el;
-        mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], NU, bas(), nc, lane);
+        mo_lap_warp<Real, PER, HL, ROWSUM, SQ_RECOMPUTE>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], NU, bas(), nc, lane);
         for (int j = lane; j < NU; j += 32) {
           vals[(size_t)el * ms + j] = double(nc[j * 5]);
           Real* mv = mov() + ((size_t)e * ms + j) * 4;
@@ -239,7 +241,7 @@ struct Walker {
       const int e0 = s == 0 ? 0 : S.nup;
       for (int el = 0; el < M; el++) {
         const int e = e0 + el;
-        mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], M, bas(), nc, lane);
+        mo_lap_warp<Real, PER, HL, ROWSUM, SQ_RECOMPUTE>(S, mocs(s), Rp[3 * e], Rp[3 * e + 1], Rp[3 * e + 2], M, bas(), nc, lane);
         for (int i = lane; i < M; i += 32) {
           aug[el * 2 * M + i] = double(nc[i * 5]);
           Real* mv = mov() + ((size_t)e * MS() + i) * 4;
@@ -336,7 +338,7 @@ struct Walker {
     if (multi()) {
       // ratios of every distinct spin-determinant (kept in mdr for accept),
       // combined with the expansion weights
-      mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), px, py, pz, S.nmo_u[s], bas(), nc, lane);
+      mo_lap_warp<Real, PER, HL, ROWSUM, SQ_PROPOSE>(S, mocs(s), px, py, pz, S.nmo_u[s], bas(), nc, lane);
       double* rr = mdr();
       for (int u = lane; u < S.nud[s]; u += 32) {
         const Real* iv = inv_u(s, u) + (size_t)el * MS();
@@ -393,7 +395,7 @@ struct Walker {
           from_gemm = true;
         }
       }
-      if (!from_gemm) mo_lap_warp<Real, PER, HL, ROWSUM>(S, mocs(s), px, py, pz, M, bas(), nc, lane);
+      if (!from_gemm) mo_lap_warp<Real, PER, HL, ROWSUM, SQ_PROPOSE>(S, mocs(s), px, py, pz, M, bas(), nc, lane);
       QWG_PHASE_END(t_mo, PH_MO, ph)
       const Real* iv = inv(s) + (size_t)el * MS();
       for (int i = 0; i < M; i++) {

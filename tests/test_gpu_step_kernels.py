@@ -1,11 +1,13 @@
 """The fused step kernel (VMC blocks, QWG_DMC_SCHEDULE=fused) and the
-shared-memory kernels on cells whose basis lists its shells in any order."""
+shared-memory kernels on periodic cells."""
+import hashlib
 import os
 import re
 
 import numpy as np
 import pytest
 
+from conftest import GOLDEN
 from mainline_b200 import engine, systems
 from test_gpu_image_sums import SHELLS, _cell, _rel
 
@@ -64,3 +66,21 @@ def test_fused_steps_do_not_depend_on_the_shell_order(kind, family, tmp_path, mo
         E.close()
     for a, b in zip(*out):
         assert _rel(a, b) < 1e-9
+
+
+def test_vmc_walk_of_a_cell_keeps_its_bits():
+    """Three VMC steps (FP64, e-e-n Jastrow, fused step kernel) against walkers
+    stored when the walk was pinned.  The orbital tables come from the host's
+    exp, so the stored walk holds where the tables are bit for bit the same."""
+    deck = os.path.join(GOLDEN, "diamond8.qw")
+    g = np.load(os.path.join(GOLDEN, "vmc_walk_cell.npz"))
+    h = hashlib.sha256()
+    for k in range(engine.inspect_deck(deck).nshell):
+        h.update(engine.inspect_spline(deck, k)[0].tobytes())
+    if h.hexdigest() != str(g["tables"]):
+        pytest.skip("this host's exp gives other orbital tables")
+    E = engine.Engine(deck, engine.FP64, max_walkers=16)
+    E.set_walkers(g["R0"])
+    E.vmc_block(3, 0.3, seed=5)
+    assert np.array_equal(E.get_walkers(), g["R"])
+    E.close()
