@@ -1009,15 +1009,12 @@ __device__ void basis_lap_team(const DevSys<Real>& S, double px, double py, doub
   tm.sync();
 }
 
-// MO value, gradient and Laplacian of one position, warp-cooperative: the
-// basis rows (basis_lap_team) in bas [nbasis][5] as Real, then lanes split
-// the (MO, component) outputs of the contraction with the MO coefficients
-// moc_s [nbasis][mstride].
-template <typename Real, int PER, bool HL = false, bool ROWSUM = false, int SQ = 0>
-__device__ void mo_lap_warp(const DevSys<Real>& S, const Real* moc_s, double px, double py, double pz, int M,
-                            Real* bas, Real* out, int lane) {
-  basis_lap_team<Real, PER, HL, ROWSUM, SQ>(S, px, py, pz, bas, WarpTeam{lane});
-  __syncwarp();
+// Contraction of the basis rows bas [nbasis][5] of one position with the MO
+// coefficients moc_s [nbasis][mstride], warp-cooperative: lanes split the
+// (MO, component) outputs.
+template <typename Real>
+__device__ __forceinline__ void mo_contract(const DevSys<Real>& S, const Real* moc_s, int M, const Real* bas, Real* out,
+                                            int lane) {
   if (M > 32) {
     // many orbitals: lanes over MOs (coalesced coefficient rows), the basis
     // values are warp-uniform reads
@@ -1061,6 +1058,25 @@ __device__ void mo_lap_warp(const DevSys<Real>& S, const Real* moc_s, double px,
     out[mo * 5] = a0; out[mo * 5 + 1] = a1; out[mo * 5 + 2] = a2; out[mo * 5 + 3] = a3; out[mo * 5 + 4] = a4;
   }
   __syncwarp();
+}
+
+// MO value, gradient and Laplacian of one position, warp-cooperative: the
+// basis rows (basis_lap_team) in bas [nbasis][5] as Real, then their
+// contraction.
+template <typename Real, int PER, bool HL = false, bool ROWSUM = false, int SQ = 0>
+__device__ void mo_lap_warp(const DevSys<Real>& S, const Real* moc_s, double px, double py, double pz, int M,
+                            Real* bas, Real* out, int lane) {
+  basis_lap_team<Real, PER, HL, ROWSUM, SQ>(S, px, py, pz, bas, WarpTeam{lane});
+  __syncwarp();
+  mo_contract(S, moc_s, M, bas, out, lane);
+}
+// The same without a call (Walker::INLINE_ROWS).
+template <typename Real, int PER, bool HL>
+__device__ __forceinline__ void mo_lap_inline(const DevSys<Real>& S, const Real* moc_s, double px, double py,
+                                              double pz, int M, Real* bas, Real* out, int lane) {
+  basis_lap_team<Real, PER, HL>(S, px, py, pz, bas, WarpTeam{lane});
+  __syncwarp();
+  mo_contract(S, moc_s, M, bas, out, lane);
 }
 
 // Cubic spline value at offset h from the row's 4 coefficients c (16-byte

@@ -77,6 +77,10 @@ struct Walker {
   // cell (mixed, 1024 walkers) takes 46.1 ms with the tables and 49.5 without,
   // that of a 32-electron cell 4.4 ms either way, in FP64 4.9 against 4.4
   static constexpr bool TBXM = TBX && sizeof(Real) == 4;
+  // MO rows of a proposal without a call in the move kernel of the HBM-resident
+  // walkers: as a call they cost it its registers (43-electron molecule, 1000
+  // walkers: 1.96 ms against 1.38 mixed, 2.61 against 2.01 in FP64)
+  static constexpr bool INLINE_ROWS = MMAX == 0 && TEAM;
   static constexpr bool CPX = MMAX < 0;
   // F and G basis shells and CUTOFF_MO: compiled into the HBM-resident kernels only
   static constexpr bool HL = MMAX < 0 || (MMAX == 0 && XL);
@@ -338,7 +342,8 @@ struct Walker {
     if (multi()) {
       // ratios of every distinct spin-determinant (kept in mdr for accept),
       // combined with the expansion weights
-      mo_lap_warp<Real, PER, HL, ROWSUM, SQ_PROPOSE>(S, mocs(s), px, py, pz, S.nmo_u[s], bas(), nc, lane);
+      if constexpr (INLINE_ROWS) mo_lap_inline<Real, PER, HL>(S, mocs(s), px, py, pz, S.nmo_u[s], bas(), nc, lane);
+      else mo_lap_warp<Real, PER, HL, ROWSUM, SQ_PROPOSE>(S, mocs(s), px, py, pz, S.nmo_u[s], bas(), nc, lane);
       double* rr = mdr();
       for (int u = lane; u < S.nud[s]; u += 32) {
         const Real* iv = inv_u(s, u) + (size_t)el * MS();
@@ -395,7 +400,10 @@ struct Walker {
           from_gemm = true;
         }
       }
-      if (!from_gemm) mo_lap_warp<Real, PER, HL, ROWSUM, SQ_PROPOSE>(S, mocs(s), px, py, pz, M, bas(), nc, lane);
+      if (!from_gemm) {
+        if constexpr (INLINE_ROWS) mo_lap_inline<Real, PER, HL>(S, mocs(s), px, py, pz, M, bas(), nc, lane);
+        else mo_lap_warp<Real, PER, HL, ROWSUM, SQ_PROPOSE>(S, mocs(s), px, py, pz, M, bas(), nc, lane);
+      }
       QWG_PHASE_END(t_mo, PH_MO, ph)
       const Real* iv = inv(s) + (size_t)el * MS();
       for (int i = 0; i < M; i++) {
