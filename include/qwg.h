@@ -7,6 +7,10 @@
  * exceptions cross this boundary.  Host buffers are caller-owned; device
  * memory is owned by the context.
  *
+ * Results do not depend on the order of calls or on other contexts.  The last
+ * bits of a walker's energies depend on the number of walkers, which decides
+ * how many warps share its sums (mixed precision: to FP32 rounding).
+ *
  * Reference interfaces each entry point replaces (QWalk/mainline src/):
  *   qwg_create          System / Pseudopotential / Wavefunction_data factories
  *                       driven by the input file: allocate(System)

@@ -77,8 +77,8 @@ struct DevSys {
   // the shells as the lanes of the basis rows take them: by shape, the longest
   // first, so that a warp's lanes run alike (the two-atom molecule's 36 shells
   // are a round of every shape and one of four S shells, which then skips the
-  // long D and P branches: move kernel, mixed, 0.32 -> 0.29 ms together with
-  // the quotients and index divisions saved in propose and accept)
+  // long D and P branches: move kernel, mixed, 0.32 -> 0.30 ms together with
+  // the index divisions saved in accept)
   const int4* shell_i;           // (center, sym, first, k)
   const int2* shell_obj;         // (table base in 4-tuples, splines in the object)
   const double* shell_cut;       // [nshell], in the order of shell_pack
@@ -1463,9 +1463,6 @@ __device__ void mo_lap_warp_cpx(const DevSys<Real>& S, const Real* moc_re, const
   __syncwarp();
 }
 
-// Determinant ratio of one electron moved to p, by the calling lane, with
-// the projected coefficients w (complex, planar with imaginary plane at
-// w_im): sum_f b_f(p) w_f over the k-phased image sums of every shell.
 // center_dot_sp with the images' k-point factors: complex sums and a complex
 // dot (each sum in image order, the functions in order); one distance per image
 // instead of one per image and shell.  Local-energy kernel of a 32-electron
@@ -1543,6 +1540,10 @@ __device__ __forceinline__ void center_dot_sp_cpx(const DevSys<Real>& S, int c, 
   }
 }
 
+// Determinant ratio of one electron moved to p, by the calling lane, with
+// the projected coefficients w (complex, planar with imaginary plane at
+// w_im): sum_f b_f(p) w_f over the k-phased image sums of every shell.  The
+// fused step kernel takes the register sums here too: energies, not moves.
 template <typename Real>
 __device__ __forceinline__ void basis_dot_lane_cpx(const DevSys<Real>& S, double px, double py, double pz,
                                                    const Real* w_re, const Real* w_im, Real& out_re, Real& out_im) {
@@ -1861,7 +1862,7 @@ __device__ void tb_pair_move(const DevSys<Real>& S, const NearSet& nsn, const Ne
 // lane pairs the moved electron with another one, so the tables replace
 // QWG_NEAR x functions radials per lane by one per entry and warp.
 struct TBMove {
-  int n[2];                 // atoms in range, -1: more than QWG_NEAR
+  int n[2];                 // atoms in range
   int a[2][QWG_NEAR];
   double d[2][QWG_NEAR][3];
   double r[2][QWG_NEAR];
@@ -1899,7 +1900,7 @@ __device__ bool tb_move_tables(const DevSys<Real>& S, const double p0[3], const 
       n += __popc(m);
     }
     if (n > QWG_NEAR) fits = false;
-    if (lane == 0) M.n[side] = n > QWG_NEAR ? -1 : n;
+    if (lane == 0) M.n[side] = n;
   }
   __syncwarp();
   if (!fits) return false;
@@ -2119,7 +2120,7 @@ __device__ void en_table_fill(const DevSys<Real>& S, const double* R, EnTable<T>
     for (int k = 0; k < S.ei_n[t]; k++) v[k] = radial_val<T>(S.ei[t][k], r);
   }
 }
-// The range bits, after en_table_fill and a synchronisation (a thread per electron).
+// The range bits, a thread per electron.
 template <typename T, typename Real>
 __device__ void en_table_near(const DevSys<Real>& S, const double* R, EnTable<T> E, int rank, int size) {
   for (int j = rank; j < S.nelec; j += size) {

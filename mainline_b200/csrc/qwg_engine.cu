@@ -740,7 +740,11 @@ static void ensure_smem_attr(K kern, size_t bytes) {
 // ms; 72-electron molecule, mixed, 2048 walkers 5.7 / 5.2 / 5.1 ms; a
 // 20-electron molecule, mixed, 4096 walkers 0.59 / 0.61 / 0.66 ms; evaluation
 // of a 43-electron molecule, mixed, 1000 walkers (its recompute is one warp's
-// work) 4.9 / 3.7 / 4.1 ms.
+// work) 4.9 / 3.7 / 4.1 ms.  At 512 walkers, local energy: 32-electron cell,
+// FP64, 7.1 / 4.0 / 2.7 ms; 128-electron cell, mixed, 30.2 / 16.7 / 10.8 ms;
+// 24-electron molecule, mixed, 0.45 / 0.27 / 0.18 ms; 72-electron molecule,
+// FP64, 5.9 / 3.3 / 2.0 ms; at 64 walkers 3.5, 3.4, 2.6 and 3.5 times faster
+// with 4 warps than with 1.
 constexpr int kWarpSlots = 148 * 16;
 static int team_warps(const qwg_ctx* c, int mode, const StepParams& P, int nwalk) {
   if (!(mode == KM_ELOC || mode == KM_ELOC_TM || mode == KM_EVAL || (mode == KM_SWEEP && P.tc_phase == 1))) return 1;

@@ -10,7 +10,9 @@ namespace qwg {
 // KM_STEPS runs whole steps (moves + local energy + weight) in one launch;
 // KM_SWEEP and KM_ELOC split one step into its two phases (the electron
 // moves; the local energy and weight), one launch each, with the same
-// arithmetic and random streams, so the two schedules give identical walks.
+// random streams and, for molecules, the same arithmetic, so that the two
+// schedules give identical walks there; on cells KM_STEPS keeps other image
+// sums (basis_lap_team) and the walks part by roundings.
 // KM_TMOVE applies the T-moves the local-energy kernel selected.
 // KM_ELOC_TM is KM_ELOC with the T-move selection compiled in.
 enum KMode { KM_EVAL = 0, KM_RATIO = 1, KM_STEPS = 2, KM_SWEEP = 3, KM_ELOC = 4, KM_TMOVE = 5, KM_ELOC_TM = 6 };
@@ -50,9 +52,10 @@ struct alignas(16) Quad { Real x[4]; };
 // XL: the F/G-shell and CUTOFF_MO code (HBM-resident kernels; the FP32 ones
 // are also compiled without it for the decks that need none, as that code's
 // register demand costs the move kernel ~5% in spills).
-// ROWSUM: see basis_lap_team (the shared-memory kernels always, which only a
-// deck forced onto them brings a periodic cell).  TEAM: the walker's threads are a CtaTeam in the
-// local energy and the evaluation (moves and recomputes are one warp's work).
+// ROWSUM: see basis_lap_team (the shared-memory kernels always: they meet a
+// periodic cell only where a deck is forced onto them).  TEAM: the walker's
+// threads are a CtaTeam in the local energy and the evaluation (moves and
+// recomputes are one warp's work).
 template <typename Real, int MMAX, bool TB, int PER, bool XL = (MMAX <= 0), bool ROWSUM = false, bool TEAM = false>
 struct Walker {
   const DevSys<Real>& S;
